@@ -33,12 +33,12 @@ constexpr int kTagSpan = 1024;                   // the clusters a tile names li
 constexpr unsigned kRecRuns = 0, kRecSame = 1, kRecOther = 2;
 
 struct __align__(16) TileRecord {
-    unsigned head;                               // kind | groups << 8 | some slot is absent << 16
+    unsigned head;                               // kind | groups << 8 | some slot is absent << 16 | an odd number of groups in a list << 17
     unsigned unused;
     unsigned short cl[kMaxU];                    // runs: the clusters (behind the last one: 0)
     union {
         unsigned char map[kTR][kMaxU];           // [row][group]: place of the group in the row + 1, 0: not named by it
-        unsigned short lists[2][kGroupMaxM];     // same: source rows by slot (0xffff: absent)
+        unsigned short lists[2][kGroupMaxM];     // same: source rows by slot (0xffff: absent, and so are the slots behind the last group)
     };
 };
 static_assert(sizeof(TileRecord) == 512, "one 16-byte piece per lane");
@@ -203,6 +203,10 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
     hole = __any_sync(kFull, hole);
     __syncwarp();
     if (same) {
+        // groups are taken in pairs, so that of an odd number of them one more is looked at: absent slots (and not the places that
+        // the attempt above may have left here)
+        if (lane < (int)sizeof(rec.lists) / 16) reinterpret_cast<uint4*>(rec.lists)[lane] = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+        __syncwarp();
 #pragma unroll
         for (int k = 0; k < 2 * RMAX; ++k) {
             const int y = g + 8 * k;
@@ -210,7 +214,7 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
             if (y < nruns && (row & 7) == 0) reinterpret_cast<unsigned*>(rec.lists[row >> 3])[4 * r + t] = pr[k];
         }
     }
-    if (lane == 0) rec.head = same ? (kRecSame | (unsigned)R << 8 | (hole ? 1u << 16 : 0u)) : kRecOther;
+    if (lane == 0) rec.head = same ? (kRecSame | (unsigned)R << 8 | (hole ? 1u << 16 : 0u) | (unsigned)(R & 1) << 17) : kRecOther;
     __syncwarp();
 }
 

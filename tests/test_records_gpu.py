@@ -1,0 +1,53 @@
+"""Records of a neighbour table's tiles (csrc/group_core.cuh): what they say about rows that are one list of 8k slots, k odd, and
+the operators over them.  The operands lie inside larger buffers of NaN, so that a row read from elsewhere shows."""
+import pytest
+import torch
+
+from helpers import TOL, rel_err
+from oracle import formula
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _inside(t, pad=1024):
+    """t as a part of a larger buffer of NaN, `pad` rows around it"""
+    flat = t.reshape(-1)
+    big = torch.full((flat.numel() + 2 * pad * 32,), float("nan"), dtype=t.dtype, device=t.device)
+    big[pad * 32:pad * 32 + flat.numel()] = flat
+    return big[pad * 32:pad * 32 + flat.numel()].view(t.shape)
+
+
+def _sources(idx, n):
+    """(kind, list entries) of every tile's record"""
+    from clusten import ops
+    tiles = idx.shape[0] * ((idx.shape[1] + 15) // 16)
+    rec = ops.build_groups(idx, n)[:tiles * 128].view(tiles, 128)
+    return rec[:, 0] & 0xff, (rec[:, 16:80].contiguous().view(torch.int16).int() & 0xffff).view(tiles, 2, 64)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16], ids=["float32", "bfloat16", "float16"])
+@pytest.mark.parametrize("clusters", [(0, 0, 1), (3, 1, 3, 2, 0), (2,), (5, 5, 4, 3, 2, 1, 5)])
+@pytest.mark.parametrize("n", [64, 49])
+def test_one_list_with_an_odd_number_of_groups(lib, clusters, n, dtype):
+    from clusten import CLUSTENAVFunction, CLUSTENQKFunction, ops
+    b, h, m = 1, 2, 8 * len(clusters)
+    row = torch.cat([torch.arange(8 * c, 8 * c + 8) for c in clusters])
+    idx = row.view(1, 1, m).expand(b, n, m).contiguous().to(DEV)
+    kind, sources = _sources(idx, n)
+    assert ((sources < n) | (sources == 0xffff) | (kind != 1).view(-1, 1, 1)).all(), "a source row that does not exist"
+    g = torch.Generator(device=DEV).manual_seed(601)
+    rn = lambda *s: _inside(torch.randn(*s, generator=g, device=DEV).to(dtype))  # noqa: E731
+    q, k, v, g_feat = (rn(b, h, n, 32) for _ in range(4))
+    attn, g_attn = rn(b, h, n, m), rn(b, h, n, m)
+    leaf = [t.detach().requires_grad_(True) for t in (q, k, attn, v)]
+    out = CLUSTENQKFunction.apply(leaf[0], leaf[1], idx), CLUSTENAVFunction.apply(leaf[2], leaf[3], idx)
+    got = out + torch.autograd.grad(out, leaf, (g_attn, g_feat))
+    want = [*formula.forward_backward("qk", q.double(), k.double(), idx, g_attn.double()),
+            *formula.forward_backward("av", attn.double(), v.double(), idx, g_feat.double())]
+    for name, x, w in zip(("attn", "feat", "d_query", "d_key", "d_attn", "d_value"), got, (want[i] for i in (0, 3, 1, 2, 4, 5))):
+        assert torch.isfinite(x).all() and rel_err(x, w) <= TOL[dtype], name
+    if m <= 48:
+        fused = ops.local_attention_forward(q, k, v, idx)
+        assert torch.isfinite(fused).all()
+        assert rel_err(fused, formula.av(formula.qk(q.double(), k.double(), idx).softmax(-1), v.double(), idx)) <= TOL[dtype], "fused"
