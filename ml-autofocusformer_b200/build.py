@@ -61,7 +61,7 @@ def _build_host(header, force, verbose):
 def build(force=False, verbose=False):
     os.makedirs(OBJ, exist_ok=True)
     sources = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
-    headers = sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + [
+    headers = sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h"))) + [
         os.path.join(HERE, "..", "include", "clusten_b200.h")]
     flags = NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else [])
 

@@ -389,7 +389,7 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
         }
         stage_rows<T, RT, SHIFT>(A + (long long)h0 * p.a_head, p.a_row, rows, m, p.R, tile, lane);
     }
-    unpack_record(sm, lane);
+    unpack_record(sm, rows, lane);
     const unsigned head = sm.rec.head;
     const unsigned kind = head & 0xffu;
     const bool holes = (head >> 16) != 0u;

@@ -20,6 +20,7 @@
 //   other   anything else: the consumer reads the indices itself, a few rows at a time (load_piece)
 #pragma once
 
+#include "index_arithmetic.h"
 #include "tile_core.cuh"
 
 namespace clusten {
@@ -219,9 +220,9 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
 }
 
 // ----------------------------------------------------------------------------- groups of a tile, for its consumers
-// The record in sm.rec -> what the products read.  "same": the lists move to sm.tok, and every row's groups are
-// 0 .. R - 1 of its list.
-__device__ __forceinline__ void unpack_record(GroupSmem& sm, int lane) {
+// The record in sm.rec -> what the products read.  "same": the lists move to sm.tok, and the groups of every row that exists
+// (`rows` of them) are 0 .. R - 1 of its list.
+__device__ __forceinline__ void unpack_record(GroupSmem& sm, int rows, int lane) {
     __syncwarp();
     if ((sm.rec.head & 0xffu) == kRecSame) {
         const uint2 v = reinterpret_cast<const uint2*>(sm.rec.lists)[lane];
@@ -229,11 +230,7 @@ __device__ __forceinline__ void unpack_record(GroupSmem& sm, int lane) {
         reinterpret_cast<uint2*>(sm.tok)[lane] = v;
         const int R = (sm.rec.head >> 8) & 0xffu;
         for (int z = lane; z < kTR * kMaxU / 4; z += 32) {
-            const int w = 4 * (z % (kMaxU / 4));
-            unsigned b = 0u;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) b |= (w + i < R ? (unsigned)(w + i + 1) : 0u) << (8 * i);
-            reinterpret_cast<unsigned*>(sm.rec.map)[z] = b;
+            reinterpret_cast<unsigned*>(sm.rec.map)[z] = list_places(z / (kMaxU / 4), 4 * (z % (kMaxU / 4)), R, rows);
         }
         __syncwarp();
     }

@@ -96,6 +96,23 @@ def test_on_model_style_views_and_against_the_separate_operators(lib, dtype):
     assert rel_err(got, sep) <= 2 * TOL[dtype]
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["float32", "bfloat16"])
+@pytest.mark.parametrize("n", [49, 41, 9])
+def test_dense_bias_at_the_end_of_a_buffer(lib, n, dtype):
+    """Shared rows, a last tile with few rows: the biases lie at the end of a larger buffer, infinite behind them."""
+    from clusten import ops
+    b, h, m, c = 2, 3, 40, 32
+    idx = workloads.make_index("shared", b, n, min(m, n), 420).to(DEV)
+    m = idx.shape[2]
+    g = torch.Generator(device=DEV).manual_seed(421)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV).to(dtype)  # noqa: E731
+    q, k, v = rn(b, h, n, c) * c ** -0.5, rn(b, h, n, c), rn(b, h, n, c)
+    big = torch.full((b * h * n * m + 16 * m,), float("inf"), dtype=dtype, device=DEV)
+    bias = big[:b * h * n * m].view(b, h, n, m).copy_(rn(b, h, n, m))
+    got = ops.local_attention_forward(q, k, v, idx, bias)
+    assert rel_err(got, _chain(q, k, v, idx, bias)) <= TOL[dtype]
+
+
 def test_argument_checks(lib):
     p = 256
     call = lib.clusten_local_attention_forward
