@@ -92,7 +92,7 @@ group_inverse_kernel(const TileRecord* __restrict__ plan, int n_rows, int m, int
             local += c;
             local_l += (cnt[T] + 15) >> 4;
         }
-        // (both sums travel in one word: fewer than 2^16 pairs and steps, else the ordinary build)
+        // (both sums travel in one word: pair_counts_fit)
         unsigned incl = (unsigned)local | (unsigned)local_l << 16;
         const unsigned mine = incl;
 #pragma unroll
@@ -226,7 +226,7 @@ int launch_group_inverse(const int64_t* idx, const void* plan, int b, int n_rows
     int words = (nlists + 31) / 32;
     size_t smem = ((size_t)ntiles * words + 2 * (size_t)ntiles) * sizeof(int);
     // too many rows for the bit mask, or so few that the entries might not fit their place: the ordinary build does everything
-    if (smem > 200 * 1024 || n_rows < 16 || (long long)n_rows * ((m + 7) / 8) > 65535) {
+    if (smem > 200 * 1024 || n_rows < 16 || !pair_counts_fit(n_rows, m)) {
         words = 0;
         smem = 0;
     }

@@ -18,4 +18,11 @@ CLUSTEN_HD unsigned list_places(int row, int first, int groups, int rows) {
     return b;
 }
 
+// Do the (source, target tile) pairs of one batch element fit the 16 bits that group_inverse_kernel counts them in?  Sources are
+// tiles of 16 rows with whole clusters (a row names at most ceil(m / 8) of them) or lists of 8 rows, of which every slot can
+// name another target tile.
+CLUSTEN_HD bool pair_counts_fit(int n_rows, int m) {
+    return (long long)n_rows * ((m + 7) / 8) <= 65535 && (long long)((n_rows + 7) / 8) * m <= 65535;
+}
+
 }  // namespace clusten

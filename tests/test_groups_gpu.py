@@ -55,3 +55,20 @@ def test_views_forward_backward(lib, kind, n, m, dtype):
     again = torch.autograd.grad((CLUSTENQKFunction.apply(leaf[0], leaf[1], idx), CLUSTENAVFunction.apply(leaf[2], leaf[3], idx)), leaf,
                                 (g_attn, g_feat))
     assert all(torch.equal(x, y) for x, y in zip(got[2:], again)), "the order of summation is fixed"
+
+
+@pytest.mark.parametrize("n,m", [(8191, 64), (8184, 64), (9361, 56)])
+def test_lists_that_name_a_target_tile_per_slot(lib, n, m):
+    """Lists whose slots are 8 tokens apart: as many (list, target tile) pairs as there are slots, at and above what the index of
+    the backward pass counts in 16 bits."""
+    from clusten import CLUSTENAVFunction
+    first = 8 * (torch.arange(n, device=DEV) // 8).view(1, n, 1)
+    idx = (first + 8 * torch.arange(m, device=DEV)) % n
+    assert (idx[:, :8] == idx[:, :1]).all()
+    g = torch.Generator(device=DEV).manual_seed(510)
+    attn, v, grad = (torch.randn(1, 1, n, w, generator=g, device=DEV) for w in (m, 32, 32))
+    leaf = attn.requires_grad_(True), v.requires_grad_(True)
+    got = torch.autograd.grad(CLUSTENAVFunction.apply(*leaf, idx), leaf, grad)
+    want = formula.forward_backward("av", attn.detach().double(), v.detach().double(), idx, grad.double())[1:]
+    for name, x, w in zip(("d_attn", "d_value"), got, want):
+        assert rel_err(x, w) <= TOL[torch.float32], name
