@@ -86,7 +86,7 @@ def host():
             raise RuntimeError("Could not load the CLUSTEN host module: " + str(e) +
                                ". Build it with `python ml-autofocusformer_b200/build.py`.") from e
         names = ("clusten_status_string", "clusten_qk_forward_views", "clusten_av_forward_views", "clusten_qk_backward_views",
-                 "clusten_av_backward_views", "clusten_local_attention_forward")
+                 "clusten_av_backward_views", "clusten_local_attention_forward", "clusten_groups_bytes", "clusten_groups_build")
         module.bind([ctypes.cast(getattr(lib, name), _p).value for name in names])
         _host = module
     return _host

@@ -22,16 +22,20 @@ struct Library {
     decltype(&clusten_qk_backward_views) qk_backward;
     decltype(&clusten_av_backward_views) av_backward;
     decltype(&clusten_local_attention_forward) local_attention;
+    decltype(&clusten_groups_bytes) groups_bytes;
+    decltype(&clusten_groups_build) groups_build;
 } lib;
 
 void bind(const std::vector<unsigned long long>& a) {
-    TORCH_CHECK(a.size() == 6, "clusten: six functions to bind");
+    TORCH_CHECK(a.size() == 8, "clusten: eight functions to bind");
     lib.status_string = reinterpret_cast<decltype(lib.status_string)>(a[0]);
     lib.qk_forward = reinterpret_cast<decltype(lib.qk_forward)>(a[1]);
     lib.av_forward = reinterpret_cast<decltype(lib.av_forward)>(a[2]);
     lib.qk_backward = reinterpret_cast<decltype(lib.qk_backward)>(a[3]);
     lib.av_backward = reinterpret_cast<decltype(lib.av_backward)>(a[4]);
     lib.local_attention = reinterpret_cast<decltype(lib.local_attention)>(a[5]);
+    lib.groups_bytes = reinterpret_cast<decltype(lib.groups_bytes)>(a[6]);
+    lib.groups_build = reinterpret_cast<decltype(lib.groups_build)>(a[7]);
 }
 
 struct Strides {                                 // of a [b, h, n, .] tensor, in elements
@@ -111,28 +115,54 @@ bool av_backward_takes(const Tensor& g, const Tensor& a, const Tensor& v, const 
     return true;
 }
 
+// Records of a table (clusten_groups_build) for one forward call.  They are made from the indices as they are now and never kept
+// for a later forward call: a table can change without a trace that could be checked (a replayed graph, another library's kernel),
+// and a buffer of another stream or of a capture need not have been written yet.
+// When they pay within the call -- QK / AV, us with the build against without: not for rows of 48, which the kernels
+// analyse at compile-time sizes (b128 h2 n3136 bf16 99 / 118 against 88 / 110, b64 h8 n196 14 / 19 against 17 / 20);  other
+// rows from 2 M scores on (b256 h16 n49 m49 39 / 36 against 46 / 41, b64 h8 n784 m24 fp32 74 / 83 against 84 / 87; below:
+// b16 h16 n49 m49 13 / 13 against 12 / 12, b4 h8 n784 m24 8 / 10 against 7 / 9).
+constexpr int64_t kRecordsMinScores = int64_t(1) << 21;
+OptTensor records(const Tensor& idx, int heads, int n, bool wanted, int& status) {
+    status = CLUSTEN_OK;
+    const int b = idx.size(0), rows = idx.size(1), m = idx.size(2);
+    if (!wanted && (m == 48 || idx.numel() * heads < kRecordsMinScores)) return std::nullopt;
+    const size_t bytes = lib.groups_bytes(b, rows, m, n);
+    if (bytes == 0) return std::nullopt;
+    Tensor groups = at::empty({(int64_t)(bytes / 4)}, idx.options().dtype(at::kInt));
+    status = launch(idx, [&](void* s) { return lib.groups_build(i64(idx), b, rows, m, n, groups.data_ptr(), bytes, s); });
+    return groups;
+}
+
 // The calls: arguments that *_takes accepted, groups and inverse from their builds.  None: sizes without a kernel.
-py::object qk_forward(const Tensor& q, const Tensor& k, const Tensor& idx, const OptTensor& groups) {
+// Forward: (result, records or None);  wanted: a backward pass will need the records.
+py::object qk_forward(const Tensor& q, const Tensor& k, const Tensor& idx, bool wanted) {
     const int b = q.size(0), h = q.size(1), n = q.size(2), m = idx.size(2);
+    int st;
+    const OptTensor groups = records(idx, h, n, wanted, st);
+    if (st != CLUSTEN_OK) fail(st);
     Tensor out = at::empty({b, h, n, m}, q.options());
-    const int st = launch(q, [&](void* s) {
+    st = launch(q, [&](void* s) {
         return lib.qk_forward(q.const_data_ptr(), Strides(q).v, k.const_data_ptr(), Strides(k).v, i64(idx), ptr(groups), out.data_ptr(), b, h, n, m,
                               32, dtype_of(q), s);
     });
     if (st == CLUSTEN_ERR_UNSUPPORTED) return py::none();
     if (st != CLUSTEN_OK) fail(st);
-    return py::cast(out);
+    return py::make_tuple(out, groups);
 }
-py::object av_forward(const Tensor& a, const Tensor& v, const Tensor& idx, const OptTensor& groups) {
+py::object av_forward(const Tensor& a, const Tensor& v, const Tensor& idx, bool wanted) {
     const int b = a.size(0), h = a.size(1), n = a.size(2), m = a.size(3);
+    int st;
+    const OptTensor groups = records(idx, h, n, wanted, st);
+    if (st != CLUSTEN_OK) fail(st);
     Tensor out = at::empty({b, h, n, 32}, a.options());
-    const int st = launch(a, [&](void* s) {
+    st = launch(a, [&](void* s) {
         return lib.av_forward(a.const_data_ptr(), Strides(a).v, v.const_data_ptr(), Strides(v).v, i64(idx), ptr(groups), out.data_ptr(), b, h, n, m,
                               32, dtype_of(a), s);
     });
     if (st == CLUSTEN_ERR_UNSUPPORTED) return py::none();
     if (st != CLUSTEN_OK) fail(st);
-    return py::cast(out);
+    return py::make_tuple(out, groups);
 }
 py::object qk_backward(const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& idx, const Tensor& groups, const Tensor& inverse) {
     const int b = q.size(0), h = q.size(1), n = q.size(2), m = idx.size(2);

@@ -1,0 +1,68 @@
+"""Buffers that the package derives from a neighbour table, and tables that change: what the operators return follows from the
+table's contents at the call."""
+import pytest
+import torch
+
+import workloads
+from helpers import TOL, rel_err
+from oracle import formula
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+SIZES = [(8, 2, 3136, 48, "model"), (24, 16, 128, 49, "shared")]           # both above 2 M scores; rows of 48 and of 49 slots
+
+
+def _operands(b, h, n, m, kind, seed):
+    first, second = (workloads.make_index(kind, b, n, m, s, DEV) for s in (seed, seed + 1))
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    q, k, v, attn = (torch.randn(b, h, n, w, generator=g, device=DEV) for w in (32, 32, 32, m))
+    return first, second, q, k, v, attn
+
+
+def _check(out, q, k, v, attn, idx):
+    assert rel_err(out[0], formula.forward("qk", q.double(), k.double(), idx, chunk=1)) <= TOL[q.dtype]
+    assert rel_err(out[1], formula.forward("av", attn.double(), v.double(), idx, chunk=1)) <= TOL[q.dtype]
+
+
+def _forward(q, k, v, attn, idx):
+    from clusten import CLUSTENAVFunction, CLUSTENQKFunction
+    return CLUSTENQKFunction.apply(q, k, idx), CLUSTENAVFunction.apply(attn, v, idx)
+
+
+@pytest.mark.parametrize("size", SIZES, ids=str)
+@pytest.mark.parametrize("grad", [False, True])
+def test_forward_after_an_untracked_write(lib, size, grad):
+    """A write that no version counter sees, as by a replayed graph or another library's kernel."""
+    idx, other, q, k, v, attn = _operands(*size, 700)
+    q.requires_grad_(grad), attn.requires_grad_(grad)
+    _forward(q, k, v, attn, idx)
+    version = idx._version
+    idx.data.copy_(other)
+    assert idx._version == version
+    _check(_forward(q, k, v, attn, idx), q.detach(), k, v, attn.detach(), other)
+
+
+@pytest.mark.parametrize("size", SIZES, ids=str)
+def test_replayed_forward_sees_new_indices(lib, size):
+    idx, other, q, k, v, attn = _operands(*size, 710)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream), torch.no_grad():
+        _forward(q, k, v, attn, idx)                         # the usual warm-up on the static inputs
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.no_grad(), torch.cuda.graph(graph, stream=stream):
+        out = _forward(q, k, v, attn, idx)
+    idx.copy_(other)
+    graph.replay()
+    _check(out, q, k, v, attn, other)
+
+
+@pytest.mark.parametrize("size", SIZES, ids=str)
+def test_forward_in_inference_mode(lib, size):
+    idx, _, q, k, v, attn = _operands(*size, 720)
+    with torch.inference_mode():
+        table = idx.clone()
+        assert table.is_inference()
+        out = _forward(q, k, v, attn, table)
+    _check(out, q, k, v, attn, idx)
