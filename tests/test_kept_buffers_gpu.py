@@ -66,3 +66,13 @@ def test_forward_in_inference_mode(lib, size):
         assert table.is_inference()
         out = _forward(q, k, v, attn, table)
     _check(out, q, k, v, attn, idx)
+
+
+def test_merge_in_inference_mode(lib):
+    from clusten import CLUSTENWFFunction
+    b, n_out, n, m, ic, c = 2, 98, 392, 48, 4, 64
+    idx = workloads.select_rows(workloads.make_index("model", b, n, m, 730), n_out, 731).to(DEV)
+    weights, feat, _ = workloads.merge_operands(b, n_out, n, m, ic, c, torch.float32, 732, DEV)
+    with torch.inference_mode():
+        out = CLUSTENWFFunction.apply(weights, feat, idx.clone())
+    assert rel_err(out, formula.forward("wf", weights.double(), feat.double(), idx)) <= TOL[torch.float32]
