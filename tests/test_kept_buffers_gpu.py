@@ -76,3 +76,40 @@ def test_merge_in_inference_mode(lib):
     with torch.inference_mode():
         out = CLUSTENWFFunction.apply(weights, feat, idx.clone())
     assert rel_err(out, formula.forward("wf", weights.double(), feat.double(), idx)) <= TOL[torch.float32]
+
+
+def test_replayed_training_step_sees_new_indices(lib):
+    """Forward and backward of all three operators, captured after a warm-up; and a call outside the graph before its first replay."""
+    from clusten import CLUSTENWFFunction
+    b, h, n, m, n_out, ic, c = 2, 2, 392, 48, 98, 4, 64
+    idx, other, q, k, v, attn = _operands(b, h, n, m, "model", 740)
+    merge, merge_other = (workloads.select_rows(t, n_out, 741) for t in (idx, other))
+    weights, feat, grad = workloads.merge_operands(b, n_out, n, m, ic, c, torch.float32, 742, DEV)
+    leaf = [t.requires_grad_(True) for t in (q, k, attn, v, weights, feat)]
+    ones = [torch.ones(b, h, n, m, device=DEV), torch.ones(b, h, n, 32, device=DEV), grad]
+
+    def step():
+        out = (*_forward(q, k, v, attn, idx), CLUSTENWFFunction.apply(weights, feat, merge))
+        return [*out, *torch.autograd.grad(out, leaf, ones)]
+
+    def check(got, table, merge_table):
+        d = [t.detach().double() for t in (q, k, attn, v, weights, feat)]
+        a, dq, dk = formula.forward_backward("qk", d[0], d[1], table, ones[0].double())
+        f, da, dv = formula.forward_backward("av", d[2], d[3], table, ones[1].double())
+        w, dw, df = formula.forward_backward("wf", d[4], d[5], merge_table, grad.double())
+        for i, (x, want) in enumerate(zip(got, (a, f, w, dq, dk, da, dv, dw, df))):
+            assert rel_err(x, want) <= TOL[torch.float32], i
+
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        out = step()
+    check(step(), idx, merge)                               # (nothing that the capture made is taken for built)
+    idx.copy_(other), merge.copy_(merge_other)
+    torch.cuda.synchronize()
+    graph.replay()
+    check(out, other, merge_other)
