@@ -35,3 +35,50 @@ def test_nothing_is_kept_or_looked_up_while_a_stream_captures(monkeypatch):
     cache.put(idx, 9, "captured")
     monkeypatch.setattr(ops, "_capturing", lambda t: False)
     assert cache.get(idx, 8) == "buffer" and cache.get(idx, 9) is None
+
+
+def test_a_buffer_belongs_to_the_stream_that_built_it(monkeypatch):
+    """Nothing orders another stream behind the build, nor the buffer's memory behind that stream's reads."""
+    from clusten import ops
+    cache, idx = _cache(), torch.zeros(1, 8, 8, dtype=torch.int64)
+    stream = [1]
+    monkeypatch.setattr(ops, "_stream_of", lambda t: stream[0])
+    cache.put(idx, 8, "first")
+    stream[0] = 2
+    assert cache.get(idx, 8) is None
+    cache.put(idx, 8, "second")
+    assert cache.get(idx, 8) == "second"
+    stream[0] = 1
+    assert cache.get(idx, 8) == "first"
+
+
+def test_threads_share_a_store():
+    """An entry found by one thread may be dropped by another before it is moved to the end."""
+    import sys
+    import threading
+    cache = _cache(1)
+    tables = [torch.zeros(1, 8, 8, dtype=torch.int64) for _ in range(4)]
+    failed, stop = [], threading.Event()
+
+    def work(k):
+        try:
+            while not stop.is_set():
+                if cache.get(tables[k], 8) is None:
+                    cache.put(tables[k], 8, k)
+                if k == 0:
+                    cache.clear()
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+            stop.set()
+
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+        [t.start() for t in threads]
+        stop.wait(2)
+        stop.set()
+        [t.join() for t in threads]
+    finally:
+        sys.setswitchinterval(interval)
+    assert not failed, failed

@@ -113,3 +113,17 @@ def test_replayed_training_step_sees_new_indices(lib):
     torch.cuda.synchronize()
     graph.replay()
     check(out, other, merge_other)
+
+
+def test_streams_have_buffers_of_their_own(lib):
+    from clusten import ops
+    idx = workloads.make_index("model", 2, 392, 48, 750, DEV)
+    torch.cuda.synchronize()
+    found = []
+    for stream in (torch.cuda.Stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(stream):
+            found.append((ops.row_order_for(idx), ops.groups_for(idx, 392)))
+            assert ops.row_order_for(idx) is found[-1][0] and ops.groups_for(idx, 392) is found[-1][1]
+    torch.cuda.synchronize()
+    assert found[0][0] is not found[1][0] and found[0][1] is not found[1][1]
+    assert torch.equal(found[0][0], found[1][0])
