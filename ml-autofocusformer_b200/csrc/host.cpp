@@ -6,6 +6,7 @@
 // serves both this module and ctypes.  Everything runs on the inputs' device and torch's current stream there.
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include "../../include/clusten_b200.h"
@@ -193,8 +194,9 @@ bool ordinary(const Tensor& t) {
     return !t._fw_grad(0).defined() && !t.key_set().has_any(c10::DispatchKeySet({DispatchKey::FuncTorchBatched, DispatchKey::FuncTorchGradWrapper,
                                                                                  DispatchKey::Functionalize, DispatchKey::Python, DispatchKey::Negative}));
 }
+// (a trace sees the operator by its node only)
 bool without_grad(const Tensor& a, const Tensor& b, const Tensor& idx) {
-    return (!at::GradMode::is_enabled() || (!a.requires_grad() && !b.requires_grad())) && ordinary(a) && ordinary(b) && ordinary(idx);
+    return !torch::jit::tracer::isTracing() && (!at::GradMode::is_enabled() || (!a.requires_grad() && !b.requires_grad())) && ordinary(a) && ordinary(b) && ordinary(idx);
 }
 
 bool dense(const OptTensor& t, const Tensor& like, at::ScalarType type, at::IntArrayRef shape) {
