@@ -72,3 +72,15 @@ def test_lists_that_name_a_target_tile_per_slot(lib, n, m):
     want = formula.forward_backward("av", attn.detach().double(), v.detach().double(), idx, grad.double())[1:]
     for name, x, w in zip(("d_attn", "d_value"), got, want):
         assert rel_err(x, w) <= TOL[torch.float32], name
+
+
+@pytest.mark.parametrize("table,message", [(lambda t: t.int(), "int64"), (lambda t: t[0], "3 dimensions"), (lambda t: t.cpu(), "CUDA"),
+                                           (lambda t: t[:, :-1].contiguous(), "mismatch")])
+def test_tables_that_are_none(lib, table, message):
+    from clusten import CLUSTENAVFunction, CLUSTENQKFunction
+    idx = table(workloads.make_index("model", 1, 64, 48, 520, DEV))
+    q, attn = torch.zeros(1, 2, 64, 32, device=DEV), torch.zeros(1, 2, 64, 48, device=DEV)
+    with pytest.raises(RuntimeError, match=message):
+        CLUSTENQKFunction.apply(q, q, idx)
+    with pytest.raises(RuntimeError, match=message):
+        CLUSTENAVFunction.apply(attn, q, idx)
