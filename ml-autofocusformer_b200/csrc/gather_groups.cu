@@ -1,4 +1,4 @@
-// Gather side of QK / AV (head_dim 32, m <= 64):
+// Gather side of QK / AV (head_dim 32, m <= 64, in fp32 m <= 48):
 //
 //   sum   out[i,:] = sum_j W[i,j] * X[idx[i,j],:]          AV forward, d_query
 //   dot   out[i,j] = <X[idx[i,j],:], Y[i,:]>               QK forward, d_attn
@@ -535,6 +535,9 @@ int gather_groups_t(const char* label, GatherGroupsParams p, int b, cudaStream_t
 
 bool gather_supported(int dtype, std::initializer_list<const void*> ptrs, int n, int m, int c) {
     if (c != kC || m < 1 || m > kGroupMaxM || n < 1 || n > 65000) return false;
+    // fp32 rows of more than 48: the plain FMAs of generic.cu, whose error against 64 bits is 1.0e-7 .. 1.4e-7 where three TF32 passes
+    // have 4.6e-7 .. 7.8e-7 (2-norm, n49 m49 .. n64 m64).  They are slower: b256 h16 n49 m49 350 / 292 us for QK / AV against 88 / 78.
+    if (dtype == CLUSTEN_F32 && m > kMmax) return false;
     if (dtype != CLUSTEN_F32 && dtype != CLUSTEN_F16 && dtype != CLUSTEN_BF16) return false;
     for (const void* p : ptrs)
         if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return false;

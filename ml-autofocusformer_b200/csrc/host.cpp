@@ -79,10 +79,10 @@ bool row_view(const Tensor& t) {
 bool rows(const Tensor& t) {
     return t.is_cuda() && t.dim() == 4 && (t.stride(3) == 1 || t.size(3) == 1) && t.stride(0) >= 0 && t.stride(1) >= 0 && t.stride(2) > 0;
 }
-// the table of rows of width 1 .. 64;  its sizes are checked separately (what is no table at all the caller's checks name)
+// the table of rows of width 1 .. 64 (fp32: 48);  its sizes are checked separately (what is no table at all the caller's checks name)
 bool table(const Tensor& first, const Tensor& second, const Tensor& idx) {
     return first.scalar_type() == second.scalar_type() && (first.scalar_type() == at::kFloat || first.scalar_type() == at::kHalf || first.scalar_type() == at::kBFloat16) &&
-           idx.is_cuda() && idx.dim() == 3 && idx.scalar_type() == at::kLong && idx.size(2) >= 1 && idx.size(2) <= 64 && idx.is_contiguous();
+           idx.is_cuda() && idx.dim() == 3 && idx.scalar_type() == at::kLong && idx.size(2) >= 1 && idx.size(2) <= (first.scalar_type() == at::kFloat ? 48 : 64) && idx.is_contiguous();
 }
 bool table_of(const Tensor& idx, const Tensor& like, int64_t b, int64_t n, int64_t m) {
     return idx.dim() == 3 && idx.size(0) == b && idx.size(1) == n && idx.size(2) == m && idx.scalar_type() == at::kLong && idx.device() == like.device();

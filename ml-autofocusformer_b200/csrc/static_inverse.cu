@@ -77,9 +77,7 @@ extern "C" int clusten_av_backward_noalloc(const void* d_feat, const void* attn,
     if (group_bytes != 0 && group_bytes <= kStaticGroupInts * sizeof(int) && dtype != CLUSTEN_F64 && c == 32) {
         int* groups = inverse + CLUSTEN_NOALLOC_MAX_INTS;
         const long long rows[3] = {(long long)h * n * m, (long long)n * m, m}, vecs[3] = {(long long)h * n * c, (long long)n * c, c};
-        const uintptr_t any = reinterpret_cast<uintptr_t>(d_feat) | reinterpret_cast<uintptr_t>(value) |
-                              reinterpret_cast<uintptr_t>(d_attn) | reinterpret_cast<uintptr_t>(d_value);
-        if (any % 16 == 0) {
+        if (clusten::tiled_dot_supported(dtype, d_feat, value, d_attn, n, m, c) && reinterpret_cast<uintptr_t>(d_value) % 16 == 0) {
             st = clusten_groups_build(nbhd_idx, b, n, m, n, groups, group_bytes, stream);
             if (st != CLUSTEN_OK) return st;
             st = clusten_inverse_build_grouped(nbhd_idx, groups, b, n, m, n, inverse, (size_t)CLUSTEN_NOALLOC_MAX_INTS * sizeof(int), stream);
