@@ -180,6 +180,61 @@ __device__ __forceinline__ void sum_head(const T* __restrict__ x, unsigned x_row
     }
 }
 
+// fp32 rows of their own (tables without locality), m <= 48: a lane takes 4 channels of every fourth neighbour, so that a load brings four
+// neighbour rows, and the next row's indices and weights travel meanwhile.  Plain FMAs: 2-norm error against 64 bits 1e-7, where
+// the TF32 passes have 6.6e-7.  src, w, out: the tile's first row;  x: the head's rows
+__device__ __noinline__ void sum_walk(const int64_t* __restrict__ src, const float* __restrict__ w, int a_row, const char* __restrict__ x, unsigned x_row,
+                                      float* __restrict__ out, int rows, int m, int n, int lane) {
+    const int q = lane >> 3;
+    x += 16 * (lane & 7);
+    int tok[2];                                              // slots lane, lane + 32 (-1: absent, its weight 0)
+    float my_w[2];
+    auto load = [&](int row) {
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+            const int j = lane + 32 * z;
+            const long long v = row < rows && j < m ? __ldg(src + (long long)row * m + j) : -1;
+            const bool there = (unsigned long long)v < (unsigned long long)n;
+            tok[z] = there ? (int)v : -1;
+            my_w[z] = there ? __ldg(w + (long long)row * a_row + j) : 0.f;
+        }
+    };
+    load(0);
+    for (int row = 0; row < rows; ++row) {
+        const int t0 = tok[0], t1 = tok[1];
+        const float w0 = my_w[0], w1 = my_w[1];
+        load(row + 1);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j0 = 0; j0 < kMmax; j0 += 16) {
+            if (j0 >= m) break;
+            float4 xv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int t = __shfl_sync(kFull, j0 < 32 ? t0 : t1, ((j0 + 4 * i) & 31) + q);
+                xv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (t >= 0) xv[i] = __ldg(reinterpret_cast<const float4*>(x + (unsigned long long)(unsigned)t * x_row));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float wv = __shfl_sync(kFull, j0 < 32 ? w0 : w1, ((j0 + 4 * i) & 31) + q);
+                acc.x += wv * xv[i].x;
+                acc.y += wv * xv[i].y;
+                acc.z += wv * xv[i].z;
+                acc.w += wv * xv[i].w;
+            }
+        }
+#pragma unroll
+        for (int o = 8; o < 32; o <<= 1) {
+            acc.x += __shfl_xor_sync(kFull, acc.x, o);
+            acc.y += __shfl_xor_sync(kFull, acc.y, o);
+            acc.z += __shfl_xor_sync(kFull, acc.z, o);
+            acc.w += __shfl_xor_sync(kFull, acc.w, o);
+        }
+        if (q == 0) st4(out + (long long)row * kC + 4 * lane, acc);
+    }
+}
+
 // ----------------------------------------------------------------------------- dot
 // Scores of rows whose length is no multiple of 8 lie in the tile as they will in the output, row after row and starting as
 // far behind a 16-byte boundary as the output does, so that they leave as 16-byte pieces.  (Taken from the places of the usual
@@ -404,6 +459,14 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
                 __syncwarp();
                 stage_rows<T, RT, SHIFT>(Ah, p.a_row, rows, m, p.R, tile, lane);
             }
+            if constexpr (kF32) {
+                if (kind == kRecOther) {
+                    cp_async_wait<0>();                      // (the weights that were requested are not used)
+                    sum_walk(src, Ah, p.a_row, reinterpret_cast<const char*>(Xh - 4 * g), p.x_row,
+                             static_cast<float*>(p.out) + (bh * n + i0) * kC, rows, m, n, lane);
+                    continue;
+                }
+            }
             const T* w = tile + g * 8 + (SHIFT ? 0 : 2 * t);
             T* o = static_cast<T*>(p.out) + (bh * n + i0 + 2 * t) * kC + 4 * g;
             if (kind == kRecRuns) {
@@ -434,7 +497,7 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
                         const unsigned short* tok = sm.tok + e * kGroupMaxM;
                         if (holes) sum_head<Pick<false, true>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
                         else sum_head<Pick<false, false>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
-                    } else {
+                    } else if constexpr (!kF32) {
                         for (int first = 8 * e, U; first < min(rows, 8 * e + 8);) {
                             first += load_piece(src, first, rows, m, n, sm, lane, &U);
                             sum_head<Pick<false, true>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, sm.tok, U, -1, n, t, acc);

@@ -38,3 +38,10 @@ def _step(kind, b, h, n, m, seed):
 def test_rows_of_more_than_48(lib, kind, n, m):
     err = _step(kind, 4, 8, n, m, 800)
     assert max(err[k] for k in ("attn", "feat", "d_query", "d_attn")) <= PLAIN, err
+
+
+@pytest.mark.parametrize("n,m", [(1000, 48), (500, 40), (300, 13)])
+def test_sums_over_rows_of_their_own(lib, n, m):
+    """Tables without locality: d_query and the forward of AV."""
+    err = _step("random", 4, 4, n, m, 810)
+    assert max(err[k] for k in ("feat", "d_query")) <= PLAIN, err
