@@ -437,7 +437,7 @@ fused_attention_kernel(const __grid_constant__ FusedParams p) {
             // one list per 8 rows, or a few rows at a time
             for (int first = 0; first < rows;) {
                 int U = U0, take = 8;
-                if (kind == kRecOther) take = load_piece(p.idx + edge0, first, rows, m, n, sm, lane, &U);
+                if (kind == kRecOther) take = load_piece<RT>(p.idx + edge0, first, rows, m, n, p.wide_idx != 0, sm, lane, &U);
                 const unsigned short* tok = sm.tok + (kind == kRecOther ? 0 : (first >> 3) * kGroupMaxM);
                 attend<Pick<false, true>, T, B::kSet>(q, kc, vc, p.x_row, bt_h, dense, m, mbits, extra, sm, tok, U, first < 8, first >= 8, -1, n, lane, st, acc);
                 first += take;

@@ -499,7 +499,7 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
                         else sum_head<Pick<false, false>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
                     } else if constexpr (!kF32) {
                         for (int first = 8 * e, U; first < min(rows, 8 * e + 8);) {
-                            first += load_piece(src, first, rows, m, n, sm, lane, &U);
+                            first += load_piece<RT>(src, first, rows, m, n, p.wide_idx != 0, sm, lane, &U);
                             sum_head<Pick<false, true>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, sm.tok, U, -1, n, t, acc);
                         }
                     }
@@ -552,7 +552,7 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
                         else one(Pick<false, false>{}, sm.tok + e * kGroupMaxM, U0);
                     } else {
                         for (int first = 8 * e, U; first < min(rows, 8 * e + 8);) {
-                            first += load_piece(src, first, rows, m, n, sm, lane, &U);
+                            first += load_piece<RT>(src, first, rows, m, n, p.wide_idx != 0, sm, lane, &U);
                             one(Pick<false, true>{}, sm.tok, U);
                         }
                     }

@@ -237,20 +237,31 @@ __device__ __forceinline__ void unpack_record(GroupSmem& sm, int rows, int lane)
 }
 
 // Any rows: those from `first` on, as many as fit a piece (at most to row `rows`), each with its own groups.  Returns
-// the number of rows; *U their groups.
-__device__ __noinline__ int load_piece(const int64_t* __restrict__ src, int first, int rows, int m, int n_src, GroupSmem& sm,
+// the number of rows; *U their groups.  A lane reads two neighbouring slots of every row (wide: as one 16-byte load).
+template <int RT>
+__device__ __noinline__ int load_piece(const int64_t* __restrict__ src, int first, int rows, int m, int n_src, bool wide, GroupSmem& sm,
                                        int lane, int* U) {
-    const int R = (m + 7) >> 3;
+    const int R = RT > 0 ? RT : (m + 7) >> 3;
     // a piece ends with its set of 8 rows
     const int take = min(min(kMaxU / R, rows - first), 8 - (first & 7));
+    const int j = 2 * lane;
+    const int64_t* p = src + (long long)first * m + j;
+    auto token = [&](long long v) { return (unsigned long long)v < (unsigned long long)n_src ? (int)v : kSkip; };
     __syncwarp();
     for (int z = lane; z < kTR * kMaxU / 4; z += 32) reinterpret_cast<unsigned*>(sm.rec.map)[z] = 0u;
-    for (int z = lane; z < 8 * 32; z += 32) {
-        const int y = z >> 3, row = y / R, j = 8 * (y - row * R) + (z & 7);
-        long long v = -1;
-        if (row < take && j < m) v = __ldg(src + (long long)(first + row) * m + j);
-        sm.tok[z] = (unsigned long long)v < (unsigned long long)n_src ? (unsigned short)v : kSkip;
+    unsigned* tok = reinterpret_cast<unsigned*>(sm.tok) + lane;
+#pragma unroll 4
+    for (int i = 0; i < take; ++i, p += m, tok += 4 * R) {
+        longlong2 v = make_longlong2(-1, -1);
+        if (RT > 0 || wide) {
+            if (j < m) v = __ldg(reinterpret_cast<const longlong2*>(p));
+        } else {
+            if (j < m) v.x = __ldg(p);
+            if (j + 1 < m) v.y = __ldg(p + 1);
+        }
+        if (j < 8 * R) *tok = pair16(token(v.x), token(v.y));
     }
+    if (lane < 4) reinterpret_cast<unsigned*>(sm.tok)[4 * R * take + lane] = 0xffffffffu;      // (groups are taken in pairs)
     __syncwarp();
     if (lane < take * R) sm.rec.map[first + lane / R][lane] = (unsigned char)(lane % R + 1);
     __syncwarp();
