@@ -30,7 +30,7 @@ constexpr int kTR = 16;                          // rows per tile
 constexpr int kGroupMaxR = 8;                    // groups per row: m <= 64
 constexpr int kGroupMaxM = 8 * kGroupMaxR;
 constexpr int kMaxU = 28;                        // distinct groups of a record or piece
-constexpr int kTagSpan = 1024;                   // the clusters a tile names lie within so many ids of each other
+constexpr int kTagSpan = 1024;                   // tags by cluster id, from the lowest one on and modulo this
 constexpr unsigned kRecRuns = 0, kRecSame = 1, kRecOther = 2;
 
 struct __align__(16) TileRecord {
@@ -125,8 +125,13 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
     }
     lo >>= 3;
     hi >>= 3;
-    if (!__any_sync(kFull, bad != 0u) && hi - lo < kTagSpan) {
-        for (int z = lane; 16 * z <= (int)(hi - lo); z += 32)
+    if (!__any_sync(kFull, bad != 0u)) {
+        // Clusters are numbered through a table of tags.  When a tile's span more ids than it has entries (the curve along which
+        // tokens are numbered leaves and comes back), two of them may share a tag: a run that finds another cluster there
+        // sees it in rec.cl, and the tile is not of this kind.
+        const bool wide_span = hi - lo >= kTagSpan;          // uniform
+        bool shared = false;
+        for (int z = lane; 16 * z <= (int)min(hi - lo, (unsigned)kTagSpan - 1u); z += 32)
             reinterpret_cast<uint4*>(tag)[z] = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
         __syncwarp();
         constexpr int NB = (2 * RMAX + 3) / 4;               // batches of 32 runs, one per lane: run g + 8 (4 j + t)
@@ -141,7 +146,7 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
             // groups are numbered in the order in which the runs first name them
             const unsigned peers = __match_any_sync(kFull, live ? cl : 0x10000u + lane);
             const bool lead = live && (peers & ((1u << lane) - 1u)) == 0u;
-            unsigned char* mytag = tag + (live ? cl - lo : 0u);
+            unsigned char* mytag = tag + (live ? (cl - lo) & (kTagSpan - 1) : 0u);
             const bool fresh = lead && *mytag == 0xffu;
             const unsigned nb = __ballot_sync(kFull, fresh);
             const int slot = U + __popc(nb & ((1u << lane) - 1u));
@@ -154,12 +159,13 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
             __syncwarp();
             const unsigned s = live ? *mytag : 0u;
             slots |= s << (8 * j);
+            if (wide_span) shared = shared || (live && rec.cl[s] != cl);
             const int row = y / R;
             if (live) rec.map[row][s] = (unsigned char)(y - row * R + 1);
         }
         __syncwarp();
-        bool twice = U > kMaxU;
-        if (!twice) {
+        bool twice = U > kMaxU || shared;
+        if (U <= kMaxU) {
             // a row that names a cluster twice has overwritten its own entry
 #pragma unroll
             for (int j = 0; j < NB; ++j) {

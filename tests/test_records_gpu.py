@@ -3,6 +3,7 @@ the operators over them.  The operands lie inside larger buffers of NaN, so that
 import pytest
 import torch
 
+import workloads
 from helpers import TOL, rel_err
 from oracle import formula
 
@@ -51,3 +52,25 @@ def test_one_list_with_an_odd_number_of_groups(lib, clusters, n, dtype):
         fused = ops.local_attention_forward(q, k, v, idx)
         assert torch.isfinite(fused).all()
         assert rel_err(fused, formula.av(formula.qk(q.double(), k.double(), idx).softmax(-1), v.double(), idx)) <= TOL[dtype], "fused"
+
+
+def test_clusters_far_apart(lib):
+    """Tables of many tokens: neighbours lie far apart along the curve that numbers the tokens.  Whole clusters stay whole
+    clusters, also when two of a tile's share a tag (their ids are 1024 apart)."""
+    from clusten import CLUSTENAVFunction, CLUSTENQKFunction
+    n, h, m = 20000, 1, 48
+    idx = workloads.make_index("model", 1, n, m, 610, DEV)
+    assert (_sources(idx, n)[0] == 0).float().mean() > 0.99
+    idx[:, 160:192] = (idx[:, 160:192] // 8 % 800 + 1024 * (torch.arange(m, device=DEV) // 8 % 2)) * 8 + torch.arange(m, device=DEV) % 8
+    idx[:, 320:352] = (torch.tensor([7, 7 + 1024, 9, 9 + 1024, 11, 12], device=DEV).repeat_interleave(8) * 8 + torch.arange(m, device=DEV) % 8)
+    g = torch.Generator(device=DEV).manual_seed(611)
+    q, k, v, g_feat = (torch.randn(1, h, n, 32, generator=g, device=DEV) for _ in range(4))
+    attn, g_attn = (torch.randn(1, h, n, m, generator=g, device=DEV) for _ in range(2))
+    leaf = [t.requires_grad_(True) for t in (q, k, attn, v)]
+    out = CLUSTENQKFunction.apply(q, k, idx), CLUSTENAVFunction.apply(attn, v, idx)
+    got = out + torch.autograd.grad(out, leaf, (g_attn, g_feat))
+    d = [t.detach().double() for t in leaf]
+    a, dq, dk = formula.forward_backward("qk", d[0], d[1], idx, g_attn.double())
+    f, da, dv = formula.forward_backward("av", d[2], d[3], idx, g_feat.double())
+    for name, x, w in zip(("attn", "feat", "d_query", "d_key", "d_attn", "d_value"), got, (a, f, dq, dk, da, dv)):
+        assert rel_err(x, w) <= TOL[torch.float32], name
