@@ -388,7 +388,7 @@ fused_attention_kernel(const __grid_constant__ FusedParams p) {
     if (p.table) warm_l1(p.pe_idx + edge0, rows * m, lane);      // (in flight while the record is made)
     if (p.mask) warm_l1(p.mask + edge0, rows * m, lane);
     build_record<RT, TAIL>(p.idx + edge0, rows, m, p.R, n, p.wide_idx != 0, sm.rec, reinterpret_cast<unsigned char*>(tile_b), lane);
-    unpack_record(sm, rows, lane);
+    unpack_record<false>(sm, rows, lane);
     const unsigned head = sm.rec.head;
     const unsigned kind = head & 0xffu;
     const int U0 = (head >> 8) & 0xffu;

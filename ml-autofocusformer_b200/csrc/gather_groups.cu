@@ -105,7 +105,7 @@ template <typename T> __device__ __forceinline__ PairAt pair_at(const T* w, int 
     return p;
 }
 
-// One head, NS sets of 8 rows.  x: the head's rows at channel 4g (RUNS: row 2t);  w: the first set's weights at row g (SHIFT: slot 0 of the
+// One head, NS sets of 8 rows.  x: the head's rows at channel 4g (RUNS: row 2t; fp32 lists without holes: as load_rows takes them);  w: the first set's weights at row g (SHIFT: slot 0 of the
 // pieces, at: where the pairs are; else slot 2t);  map: the record's row g of the first set
 template <typename PICK, typename T, bool SHIFT, int NS, int SET>
 __device__ __forceinline__ void sum_head(const T* __restrict__ x, unsigned x_row, const T* w, const PairAt (&at)[NS], const unsigned char* map,
@@ -122,11 +122,19 @@ __device__ __forceinline__ void sum_head(const T* __restrict__ x, unsigned x_row
             if (h == 1 && u0 + 2 >= U) break;
             Four_t<T> v[4];
             unsigned tk[2];
-            load_four<PICK, T>(v, reinterpret_cast<const char*>(x), x_row, sm, tok, u0 + 2 * h, t, pad_cl, n, tk);
+            // fp32, one set of rows (lists): whole rows, as the L1 likes them, moved to their lanes (b128 h2 n3136 146 -> 138 us)
+            constexpr bool kWhole = std::is_same<T, float>::value && NS == 1 && !PICK::kRuns && !PICK::kHoles;
+            RowRegs<T> whole;
+            if constexpr (kWhole) load_rows<PICK>(whole, reinterpret_cast<const char*>(x), x_row, sm, tok, u0 + 2 * h, threadIdx.x & 31, pad_cl, n);
+            else load_four<PICK, T>(v, reinterpret_cast<const char*>(x), x_row, sm, tok, u0 + 2 * h, t, pad_cl, n, tk);
             if (!landed) {                                   // the weights travelled together with the first rows
                 cp_async_wait<0>();
                 __syncwarp();
                 landed = true;
+            }
+            if constexpr (kWhole) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = to_slots(whole.v[i], threadIdx.x & 31);
             }
             if constexpr (std::is_same<T, float>::value) {
                 auto weights = [&](int e, int i, float (&bb)[2]) {
@@ -400,11 +408,12 @@ __device__ __forceinline__ void store_rows(const T* tile, T* __restrict__ out, i
 // SHIFT: the rows of the weights (sum) or scores (dot, LinearRows) do not start on 16-byte boundaries;  PLAN: the records are there;
 // TAIL: the last cluster is padded
 // CTAs per SM, measured for b128 h2 n3136 (and b32 h8 n1843).  dot: fp32 over records 7 (0.115 ms a call, 0.130 with 5), 5 where the
-// records are made here, since those calls are small and want each warp fast; 16-bit 4, without spills (0.069 (0.056) ms,
-// 0.079 (0.069) with 6).  sum: fp32 5, 16-bit 7 (0.086 (0.068) ms, 0.089 (0.083) with 6).
+// records are made here (b4 h2 n9216 22 us, 24 with 6); 16-bit 4, without spills (0.069 (0.056) ms, 0.079 (0.069) with 6).
+// sum: fp32 over records 5, 6 where they are made here (shared tables 134 us, 138 with 5; b128 h8 n196 45, 50 with 5), 16-bit 7
+// (0.086 (0.068) ms, 0.089 (0.083) with 6).
 template <typename T, int MODE, bool PLAN> constexpr int gather_ctas() {
     if (MODE == 1) return sizeof(T) == 4 ? (PLAN ? 7 : 5) : 4;
-    return sizeof(T) == 4 ? 5 : 7;
+    return sizeof(T) == 4 ? (PLAN ? 5 : 6) : 7;
 }
 template <typename T, int MODE, int RT, bool SHIFT, bool PLAN, bool TAIL>
 __global__ void __launch_bounds__(32 * kGWarps, (gather_ctas<T, MODE, PLAN>()))
@@ -444,10 +453,12 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
         }
         stage_rows<T, RT, SHIFT>(A + (long long)h0 * p.a_head, p.a_row, rows, m, p.R, tile, lane);
     }
-    unpack_record(sm, rows, lane);
+    // (16-bit sums: 0 * Inf would be a NaN; three-pass products of infinities are NaN anyway)
+    constexpr bool kFill = MODE == 1 || kF32;
+    unpack_record<kFill>(sm, rows, lane);
     const unsigned head = sm.rec.head;
     const unsigned kind = head & 0xffu;
-    const bool holes = (head >> 16) != 0u;
+    const bool holes = (head >> 16 & (kFill ? 1u : 3u)) != 0u;
     const int U0 = (head >> 8) & 0xffu;
     auto at_row = [&](const T* x, int row) { return reinterpret_cast<const T*>(reinterpret_cast<const char*>(x) + (unsigned long long)row * p.x_row); };
     for (int h = h0; h < h1; ++h) {
@@ -496,7 +507,7 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
                     if (kind == kRecSame) {
                         const unsigned short* tok = sm.tok + e * kGroupMaxM;
                         if (holes) sum_head<Pick<false, true>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
-                        else sum_head<Pick<false, false>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
+                        else sum_head<Pick<false, false>, T, SHIFT, 1, Tile::kSet>(kF32 ? Xh - 4 * g + rows_channel<T>(lane) : Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
                     } else if constexpr (!kF32) {
                         for (int first = 8 * e, U; first < min(rows, 8 * e + 8);) {
                             first += load_piece<RT>(src, first, rows, m, n, p.wide_idx != 0, sm, lane, &U);

@@ -227,14 +227,17 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
 
 // ----------------------------------------------------------------------------- groups of a tile, for its consumers
 // The record in sm.rec -> what the products read.  "same": the lists move to sm.tok, and the groups of every row that exists
-// (`rows` of them) are 0 .. R - 1 of its list.
+// (`rows` of them) are 0 .. R - 1 of its list.  FILL: the absent group behind an odd number of them repeats a token of the list, for
+// consumers to whom a product that nobody looks at, or a zero weight, does no harm.
+template <bool FILL>
 __device__ __forceinline__ void unpack_record(GroupSmem& sm, int rows, int lane) {
     __syncwarp();
     if ((sm.rec.head & 0xffu) == kRecSame) {
-        const uint2 v = reinterpret_cast<const uint2*>(sm.rec.lists)[lane];
+        const int R = (sm.rec.head >> 8) & 0xffu;
+        uint2 v = reinterpret_cast<const uint2*>(sm.rec.lists)[lane];
+        if (FILL && 4 * (lane & 15) >= 8 * R) v.x = v.y = sm.rec.lists[lane >> 4][0] * 0x10001u;
         __syncwarp();
         reinterpret_cast<uint2*>(sm.tok)[lane] = v;
-        const int R = (sm.rec.head >> 8) & 0xffu;
         for (int z = lane; z < kTR * kMaxU / 4; z += 32) {
             reinterpret_cast<unsigned*>(sm.rec.map)[z] = list_places(z / (kMaxU / 4), 4 * (z % (kMaxU / 4)), R, rows);
         }
