@@ -328,6 +328,23 @@ __device__ __forceinline__ void mma_tf32_first(float (&d)[4], const unsigned (&a
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
 }
 
+// mma_pair of fp32 values (tile_core.cuh) whose accumulators start at zero
+__device__ __forceinline__ void mma_pair_first(float (&d)[2][4], const float (&a)[2][4], const float (&b)[2]) {
+    unsigned ah[2][4], al[2][4], bh[2], bl[2];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) split_tf32(a[mt][i], ah[mt][i], al[mt][i]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) split_tf32(b[i], bh[i], bl[i]);
+    mma_tf32_first(d[0], al[0], bh);
+    mma_tf32_first(d[1], al[1], bh);
+    mma_tf32(d[0], ah[0], bl);
+    mma_tf32(d[1], ah[1], bl);
+    mma_tf32(d[0], ah[0], bh);
+    mma_tf32(d[1], ah[1], bh);
+}
+
 // Four channels of a row, as the element type's vector
 template <typename T> struct Four { using type = uint2; };
 template <> struct Four<float> { using type = float4; };

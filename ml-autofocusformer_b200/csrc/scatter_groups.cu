@@ -48,7 +48,9 @@ __device__ __forceinline__ void step16(float (&acc)[2][4], const T* const (&r)[4
     mma16(acc[0], a[0], b, static_cast<const T*>(nullptr));
     mma16(acc[1], a[1], b, static_cast<const T*>(nullptr));
 }
-__device__ __forceinline__ void step8(float (&acc)[2][4], const float* const (&r)[2], const float* const (&w)[2]) {
+// (FIRST: d starts at zero)
+template <bool FIRST>
+__device__ __forceinline__ void step8(float (&d)[2][4], const float* const (&r)[2], const float* const (&w)[2]) {
     float4 x[2];
     float b[2];
 #pragma unroll
@@ -58,18 +60,33 @@ __device__ __forceinline__ void step8(float (&acc)[2][4], const float* const (&r
         b[i] = w[i] ? __ldg(w[i]) : 0.f;
     }
     const float a[2][4] = {{x[0].x, x[0].y, x[1].x, x[1].y}, {x[0].z, x[0].w, x[1].z, x[1].w}};
-    mma_pair<true>(acc, a, b);
+    if (FIRST) mma_pair_first(d, a, b);
+    else mma_pair<true>(d, a, b);
 }
-// rows and weights of 16 rows (4 per lane)
-template <typename T>
+// rows and weights of 16 rows (4 per lane).  ALONE, fp32: the products of a step are added up by themselves and then to the accumulator:
+// a tensor core cuts its sums off, and over the hundreds of rows that name a cluster the cut adds up (2-norm error against 64 bits
+// of d_key, d_value, straight into the accumulator and so: b8 h8 n196 7.7e-7 -> 4.5e-7, b4 h8 n1843 7.5e-7 -> 4.5e-7, b8 h2 n3136
+// 7.4e-7 -> 4.5e-7).  The lists of shared tables are short; there the extra registers cost 8 % of a training pass.
+template <typename T, bool ALONE>
 __device__ __forceinline__ void step_rows(float (&acc)[2][4], const T* const (&r)[4], const T* const (&w)[4]) {
     if constexpr (std::is_same<T, float>::value) {
         const float* const ra[2] = {r[0], r[1]};
         const float* const wa[2] = {w[0], w[1]};
         const float* const rb[2] = {r[2], r[3]};
         const float* const wb[2] = {w[2], w[3]};
-        step8(acc, ra, wa);
-        step8(acc, rb, wb);
+        if constexpr (ALONE) {
+            float d[2][4];
+            step8<true>(d, ra, wa);
+            step8<false>(d, rb, wb);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc[0][i] += d[0][i];
+                acc[1][i] += d[1][i];
+            }
+        } else {
+            step8<false>(acc, ra, wa);
+            step8<false>(acc, rb, wb);
+        }
     } else {
         step16<T>(acc, r, w);
     }
@@ -121,7 +138,7 @@ scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
                         r[i] = place ? X + (long long)row * p.x_row : nullptr;
                         w[i] = place && live ? w0 + (long long)row * p.w_row + 8 * place : nullptr;
                     }
-                    step_rows<T>(acc, r, w);
+                    step_rows<T, true>(acc, r, w);
                 }
             };
             walk(ents + (start >> 2), count >> 4, Wg, true);
@@ -153,7 +170,7 @@ scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
                     }
                 }
                 if (k + 2 < count) load(k + 2);
-                step_rows<T>(acc, r, w);
+                step_rows<T, false>(acc, r, w);
             }
         } else {
             // the ordinary index: target by target, 16 entries per step
@@ -180,7 +197,7 @@ scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
                             }
                         }
                     }
-                    step_rows<T>(acc, r, w);
+                    step_rows<T, false>(acc, r, w);
                     if (__any_sync(kFull, repeats)) {
                         // the row's weights for the target are added up in fp32, in slot order
                         for (int z = k; z < min(k + 16, len); ++z) {

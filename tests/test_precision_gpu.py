@@ -45,3 +45,10 @@ def test_sums_over_rows_of_their_own(lib, n, m):
     """Tables without locality: d_query and the forward of AV."""
     err = _step("random", 4, 4, n, m, 810)
     assert max(err[k] for k in ("feat", "d_query")) <= PLAIN, err
+
+
+# d_key and d_value over whole clusters, three TF32 passes: errors of the kernels that added up 48 rows at a time
+@pytest.mark.parametrize("b,h,n,limit", [(8, 8, 196, 6.4e-7), (4, 8, 1843, 6.6e-7), (8, 2, 3136, 7.1e-7)])
+def test_gradients_over_long_lists(lib, b, h, n, limit):
+    err = _step("model", b, h, n, 48, 3)
+    assert max(err[k] for k in ("d_key", "d_value")) <= 1.02 * limit, err
