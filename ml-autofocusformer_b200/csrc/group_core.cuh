@@ -497,6 +497,8 @@ template <typename T> __device__ __forceinline__ int rows_first(int lane) { retu
 template <typename T, int E, typename BF>
 __device__ __forceinline__ void rows_product(float (&acc)[E][2][4], const RowRegs<T>& r, int lane, BF&& bf) {
     if constexpr (std::is_same<T, float>::value) {
+        // (added up by themselves first: see step_rows in scatter_groups.cu)
+        float d[E][2][4];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const float4 x0 = to_slots(r.v[2 * i], lane), x1 = to_slots(r.v[2 * i + 1], lane);
@@ -505,9 +507,17 @@ __device__ __forceinline__ void rows_product(float (&acc)[E][2][4], const RowReg
             for (int e = 0; e < E; ++e) {
                 const float2 w = bf(e, i);
                 const float b[2] = {w.x, w.y};
-                mma_pair<true>(acc[e], a, b);
+                if (i == 0) mma_pair_first(d[e], a, b);
+                else mma_pair<true>(d[e], a, b);
             }
         }
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc[e][0][i] += d[e][0][i];
+                acc[e][1][i] += d[e][1][i];
+            }
     } else {
         unsigned a[2][4];
         frag_slots16(a, r.v[0], r.v[1]);

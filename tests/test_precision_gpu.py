@@ -52,3 +52,23 @@ def test_sums_over_rows_of_their_own(lib, n, m):
 def test_gradients_over_long_lists(lib, b, h, n, limit):
     err = _step("model", b, h, n, 48, 3)
     assert max(err[k] for k in ("d_key", "d_value")) <= 1.02 * limit, err
+
+
+@pytest.mark.parametrize("b,h,n,m", [(4, 2, 3136, 48), (4, 8, 1843, 48), (4, 4, 784, 24)])
+def test_fused_attention_with_a_blank_token(lib, b, h, n, m):
+    """The kernel before the online softmax had 9.9e-7 at m = 48, 7.8e-7 at m = 24."""
+    from clusten import ops
+    idx = workloads.make_index("model", b, n, m, 3, DEV)
+    g = torch.Generator(device=DEV).manual_seed(6)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    q, k, v = rn(b, h, n, 32) * 32 ** -0.5, rn(b, h, n, 32), rn(b, h, n, 32)
+    table, pe_idx = rn(12321, h), torch.randint(0, 12321, (b, n, m), device=DEV, generator=g)
+    blank_k, blank_v = rn(h, 32), rn(h, 32)
+    got = ops.local_attention_forward(q, k, v, idx, pe_table=table, pe_idx=pe_idx, blank_k=blank_k, blank_v=blank_v)
+    want = []
+    for i in range(b):
+        logits = formula.qk(q[i:i + 1].double(), k[i:i + 1].double(), idx[i:i + 1])[0] + table.double()[pe_idx[i]].permute(2, 0, 1)
+        blank = (q[i].double() * blank_k.double().unsqueeze(1)).sum(-1, keepdim=True)
+        p = torch.cat([logits, blank], -1).softmax(-1)
+        want.append(formula.av(p[None, ..., :m], v[i:i + 1].double(), idx[i:i + 1])[0] + p[..., m:] * blank_v.double().unsqueeze(1))
+    assert _norm_err(got, torch.stack(want)) <= (9.9e-7 if m == 48 else 7.9e-7)
