@@ -190,7 +190,11 @@ CLUSTEN_API int clusten_qk_backward(const void* d_attn, const void* query, const
                         int b, int h, int n, int m, int c, int dtype, void* stream);
 
 /* Inverse of a neighbour table by groups, for the *_backward_views calls below: same buffer size as
- * clusten_inverse_build (clusten_inverse_bytes), its own contents.  groups: clusten_groups_build on the same table. */
+ * clusten_inverse_build (clusten_inverse_bytes), its own contents.  groups: clusten_groups_build on the same table.
+ * Tables outside the range of its kernel (from about 10000 tokens on at m = 48) get the ordinary index, over which those
+ * calls go target by target: clusten_inverse_grouped_applies returns 0 for their sizes, and clusten_inverse_build with
+ * clusten_qk_backward / clusten_av_backward is the faster way. */
+CLUSTEN_API int clusten_inverse_grouped_applies(int n_rows, int m, int n_targets);
 CLUSTEN_API int clusten_inverse_build_grouped(const int64_t* nbhd_idx, const void* groups, int b, int n_rows, int m,
                                               int n_targets, void* inverse, size_t inverse_bytes, void* stream);
 

@@ -30,6 +30,7 @@ SIGNATURES = {
     "clusten_groups_build": (_i, [_p, _i, _i, _i, _i, _p, _sz, _p]),
     "clusten_qk_forward_views": (_i, [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p]),
     "clusten_av_forward_views": (_i, [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p]),
+    "clusten_inverse_grouped_applies": (_i, [_i, _i, _i]),
     "clusten_inverse_build_grouped": (_i, [_p, _p, _i, _i, _i, _i, _p, _sz, _p]),
     "clusten_qk_backward_views": (_i, [_p] * 11 + [_i, _i, _i, _i, _i, _i, _p]),
     "clusten_av_backward_views": (_i, [_p] * 11 + [_i, _i, _i, _i, _i, _i, _p]),

@@ -383,6 +383,8 @@ int clusten_av_forward_views(const void* attn, const long long* attn_strides, co
     return launch_tiled_sum("av_forward", dtype, attn, value, nbhd_idx, feat, b, h, n, m, (cudaStream_t)stream, gs, groups);
 }
 
+int clusten_inverse_grouped_applies(int n_rows, int m, int n_targets) { return group_inverse_applies(n_rows, m, n_targets) ? 1 : 0; }
+
 int clusten_inverse_build_grouped(const int64_t* nbhd_idx, const void* groups, int b, int n_rows, int m, int n_targets,
                                   void* inverse, size_t inverse_bytes, void* stream) {
     const int st = check_inverse_args(b, n_rows, m, n_targets);

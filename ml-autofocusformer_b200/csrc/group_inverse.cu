@@ -218,18 +218,22 @@ group_lists_kernel(int n_rows, int m, int nt, int ntiles, unsigned total, const 
 
 }  // namespace
 
+// Shared memory of group_inverse_kernel; 0: too many rows for the bit mask or the counters, or so few that the entries might not fit
+// their place
+static size_t group_inverse_smem(int n_rows, int m, int nt) {
+    const int ntiles = inverse_tiles(nt), words = ((n_rows + 7) / 8 + 31) / 32;
+    const size_t smem = ((size_t)ntiles * words + 2 * (size_t)ntiles) * sizeof(int);
+    return smem > 200 * 1024 || n_rows < 16 || !pair_counts_fit(n_rows, m) ? 0 : smem;
+}
+
+bool group_inverse_applies(int n_rows, int m, int nt) { return group_plan_supported(nt, m) && group_inverse_smem(n_rows, m, nt) != 0; }
+
 int launch_group_inverse(const int64_t* idx, const void* plan, int b, int n_rows, int m, int nt, void* buf, cudaStream_t s) {
     int* p = static_cast<int*>(buf);
     const InverseView v = inverse_view(buf, b, n_rows, m, nt);
     const int ntiles = inverse_tiles(nt);
-    const int nlists = (n_rows + 7) / 8;
-    int words = (nlists + 31) / 32;
-    size_t smem = ((size_t)ntiles * words + 2 * (size_t)ntiles) * sizeof(int);
-    // too many rows for the bit mask, or so few that the entries might not fit their place: the ordinary build does everything
-    if (smem > 200 * 1024 || n_rows < 16 || !pair_counts_fit(n_rows, m)) {
-        words = 0;
-        smem = 0;
-    }
+    const size_t smem = group_inverse_smem(n_rows, m, nt);
+    const int words = smem != 0 ? ((n_rows + 7) / 8 + 31) / 32 : 0;          // (0: the ordinary build does everything)
     const int fit = resident_ctas(reinterpret_cast<const void*>(group_inverse_kernel), kGIThreads, smem);
     if (fit < 0) return fit;
     {

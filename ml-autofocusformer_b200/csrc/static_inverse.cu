@@ -74,7 +74,7 @@ extern "C" int clusten_av_backward_noalloc(const void* d_feat, const void* attn,
     if (st != CLUSTEN_OK) return st;
     // the kernels of the regular operator where they apply ...
     const size_t group_bytes = clusten_groups_bytes(b, n, m, n);
-    if (group_bytes != 0 && group_bytes <= kStaticGroupInts * sizeof(int) && dtype != CLUSTEN_F64 && c == 32) {
+    if (group_bytes != 0 && group_bytes <= kStaticGroupInts * sizeof(int) && group_inverse_applies(n, m, n) && dtype != CLUSTEN_F64 && c == 32) {
         int* groups = inverse + CLUSTEN_NOALLOC_MAX_INTS;
         const long long rows[3] = {(long long)h * n * m, (long long)n * m, m}, vecs[3] = {(long long)h * n * c, (long long)n * c, c};
         if (clusten::tiled_dot_supported(dtype, d_feat, value, d_attn, n, m, c) && reinterpret_cast<uintptr_t>(d_value) % 16 == 0) {

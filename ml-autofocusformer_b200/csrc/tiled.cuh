@@ -17,6 +17,7 @@ struct GatherStrides {
 inline int group_tiles(int n_rows) { return (n_rows + 15) / 16; }
 size_t group_plan_bytes(int b, int n_rows);
 bool group_plan_supported(int n_src, int m);
+bool group_inverse_applies(int n_rows, int m, int nt);      // (group_inverse.cu)
 int launch_group_plan(const int64_t* idx, int b, int n_rows, int m, int n_src, void* plan, cudaStream_t s);
 
 // gather-sum:  out[b,h,i,:] = sum_j W[b,h,i,j] * X[b,h,idx[b,i,j],:]      (AV forward, d_query)

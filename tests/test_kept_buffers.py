@@ -82,3 +82,10 @@ def test_threads_share_a_store():
     finally:
         sys.setswitchinterval(interval)
     assert not failed, failed
+
+
+def test_tables_beyond_the_inverse_by_groups(lib):
+    """They take the way of an explicit inverse (and nothing is kept for another one)."""
+    applies = lib.clusten_inverse_grouped_applies
+    assert applies(9216, 48, 9216) and applies(196, 48, 196) and applies(3136, 64, 3136) and applies(16, 8, 16)
+    assert not applies(12800, 48, 12800) and not applies(9, 48, 9) and not applies(8191, 64, 8191) and not applies(196, 65, 196)
