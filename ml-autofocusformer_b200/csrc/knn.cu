@@ -73,7 +73,8 @@ knn2d_kernel(const float2* __restrict__ query, const float2* __restrict__ db, in
                     const float d[4] = {d0.x, d0.y, d1.x, d1.y};
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
-                        if (d[i] <= best[K - 1] && 4 * at + i < cnt) insert(d[i], t0 + 4 * at + i);
+                        // (points at an infinite distance, as padding has them, are nobody's neighbours)
+                        if (d[i] <= best[K - 1] && d[i] < CUDART_INF_F && 4 * at + i < cnt) insert(d[i], t0 + 4 * at + i);
                 }
                 at = at + 1 < quads ? at + 1 : 0;
             }

@@ -50,3 +50,15 @@ def test_argument_checks(lib):
     assert lib.clusten_knn2d(p, p, 1, 4, 3, 4, p, None, None) == -6      # k above n
     assert lib.clusten_knn2d(p, p, 0, 4, 4, 2, p, None, None) == -2
     assert lib.clusten_knn2d(None, p, 1, 4, 4, 2, p, None, None) == -3
+
+
+def test_points_at_infinity_are_nobodys_neighbours(lib):
+    """Padding at an infinite position: places that no finite point takes stay empty (2^31 - 1, an infinite distance), which the
+    tables of the neighbourhood (clusten_nbhd_build) take for nobody."""
+    from clusten import ops
+    q = torch.rand(2, 70, 2, device=DEV)
+    d = torch.full((2, 37, 2), float("inf"), device=DEV)
+    d[:, 5], d[:, 20, 0], d[:, 36] = 0.25, 0.5, 0.75
+    idx, dist = ops.knn2d(q, d, 4, return_dist=True)
+    assert (idx[..., 2:] == 2 ** 31 - 1).all() and torch.isinf(dist[..., 2:]).all()
+    assert (idx[..., :2].sort(dim=2).values == torch.tensor([5, 36], device=DEV)).all()
