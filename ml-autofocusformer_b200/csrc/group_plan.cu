@@ -1,7 +1,7 @@
 // Records of a neighbour table's tiles (group_core.cuh), one warp per tile of 16 rows.
 //
-// Every consumer of the table -- the forward and backward of QK and AV in all blocks of a stage, the fused attention --
-// then reads 512 bytes per tile instead of 6 KB of int64 indices.  Bound by the one pass over the indices.
+// The backward passes of QK and AV in all blocks of a stage, and forward calls for which that pays by itself, then read 512 bytes
+// per tile instead of 6 KB of int64 indices.  Bound by the one pass over the indices.
 #include "group_core.cuh"
 
 namespace clusten {

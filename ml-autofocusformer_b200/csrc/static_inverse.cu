@@ -6,8 +6,8 @@
 // inference engine's enqueue callback, or any program that hands all device memory to its own pool
 // up front, may neither call cudaMalloc (it can fail, and it synchronises the device) nor ask the
 // pool from inside the callback.  For them the inverse index lives in the fixed array below, which
-// every GPU that loads this library holds until the process exits (kStaticInverseInts * 4 bytes,
-// about 13.6 MB).  Nothing here allocates: no cudaMalloc / cudaFree and no allocating library call.
+// every GPU that loads this library holds until the process exits (17.8 MB with the table's
+// groups behind it).  Nothing here allocates: no cudaMalloc / cudaFree and no allocating library call.
 //
 // In host code `g_static_inverse` is only a stand-in for the device array, never a device address;
 // the address a kernel may use comes from cudaGetSymbolAddress, taken once per device, with that

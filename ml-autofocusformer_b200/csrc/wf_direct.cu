@@ -138,7 +138,7 @@ wf_forward_direct_kernel(const WfDirectParams p) {
 // registers: of the 8 x 8 block whose rows are (slot, half of the 64 channels), movmatrix leaves lane (g, t) = (lane / 4, lane % 4)
 // one channel of each half of slot t;  two such blocks, slots 0 .. 3 and 4 .. 7, are byte-permuted into the A operand, k being the
 // order 0 4 1 5 2 6 3 7 of the slots, in which the lane fetches the weights.  Bound by the L1 and what it misses:
-// b64 n9216 n_out 1843 c128 bf16 178 us, 284 in the walk above, b128 n_out 784 c64 98 us, 110 (L1 pipe 85 % busy).
+// b64 n9216 n_out 1843 c128 bf16 178 us (L1 pipe 85 % busy), 284 in the walk above, b128 n_out 784 c64 98 us, 110.
 constexpr int kFw16Warps = 4;
 struct WfFw16Params {
     const void* W;  const void* F;  void* out;
