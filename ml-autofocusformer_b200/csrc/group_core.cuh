@@ -365,8 +365,8 @@ __device__ __forceinline__ void load_four(Four_t<T> (&v)[4], const char* x, unsi
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const unsigned c = i == 0 ? cc & 0xffffu : cc >> 16;
-            const char* p0 = x + (unsigned long long)c * (8u * x_row);
-            const char* p1 = x1 + (unsigned long long)c * (8u * x_row);
+            const char* p0 = x + (unsigned long long)(8u * c) * x_row;
+            const char* p1 = x1 + (unsigned long long)(8u * c) * x_row;
             if (PICK::kTail) {                               // slots behind the last token: token 0
                 const int left = (int)c == pad_cl ? n - 8 * (int)c - 2 * t : 8;
                 const char* x0 = x - (unsigned long long)(2 * t) * x_row;
@@ -398,7 +398,7 @@ __device__ __forceinline__ const char* slot_ptr(const char* x, unsigned x_row, c
                                                 int pad_cl, int n) {
     if constexpr (PICK::kRuns) {
         const unsigned c = sm.rec.cl[u];
-        const char* p = x + (unsigned long long)c * (8u * x_row);
+        const char* p = x + (unsigned long long)(8u * c) * x_row;
         if (PICK::kTail) p = (int)c == pad_cl && 8 * (int)c + g >= n ? x - (unsigned long long)g * x_row : p;
         return p;
     } else {
@@ -466,8 +466,8 @@ __device__ __forceinline__ void load_rows(RowRegs<float>& r, const char* x, unsi
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const unsigned c = i == 0 ? cc & 0xffffu : cc >> 16;
-            const char* p0 = x + (unsigned long long)c * (8u * x_row);
-            const char* p1 = x1 + (unsigned long long)c * (8u * x_row);
+            const char* p0 = x + (unsigned long long)(8u * c) * x_row;
+            const char* p1 = x1 + (unsigned long long)(8u * c) * x_row;
             if (PICK::kTail) {                               // slots behind the last token: token 0
                 const int left = (int)c == pad_cl ? n - 8 * (int)c - 2 * q : 8;
                 const char* x0 = x - (unsigned long long)(2 * q) * x_row;

@@ -84,3 +84,18 @@ def test_tables_that_are_none(lib, table, message):
         CLUSTENQKFunction.apply(q, q, idx)
     with pytest.raises(RuntimeError, match=message):
         CLUSTENAVFunction.apply(attn, q, idx)
+
+
+def test_rows_half_a_gigabyte_apart(lib):
+    """The row stride is kept in 32 bits; eight rows of it are not."""
+    from clusten import CLUSTENAVFunction, CLUSTENQKFunction, ops
+    n, m, row = 24, 16, 1 << 28                             # bf16: 2^29 bytes
+    idx = (8 * torch.tensor([[1, 2], [2, 0], [0, 1]], device=DEV).repeat_interleave(8, 0).unsqueeze(2) + torch.arange(8, device=DEV)).view(1, n, m)
+    g = torch.Generator(device=DEV).manual_seed(530)
+    x = torch.randn(1, 1, n, 32, generator=g, device=DEV).bfloat16()
+    attn = torch.randn(1, 1, n, m, generator=g, device=DEV).bfloat16()
+    far = torch.empty((n - 1) * row + 32, dtype=torch.bfloat16, device=DEV).as_strided((1, 1, n, 32), (32, 32, row, 1)).copy_(x)
+    for got, want in ((CLUSTENQKFunction.apply(x, far, idx), CLUSTENQKFunction.apply(x, x, idx)),
+                      (CLUSTENAVFunction.apply(attn, far, idx), CLUSTENAVFunction.apply(attn, x, idx)),
+                      (ops.local_attention_forward(x, far, far, idx), ops.local_attention_forward(x, x, x, idx))):
+        assert torch.equal(got, want)
