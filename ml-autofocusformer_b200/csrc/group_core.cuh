@@ -36,7 +36,7 @@ constexpr unsigned kRecRuns = 0, kRecSame = 1, kRecOther = 2;
 struct __align__(16) TileRecord {
     unsigned head;                               // kind | groups << 8 | some slot is absent << 16 | an odd number of groups in a list << 17
     unsigned unused;
-    unsigned short cl[kMaxU];                    // runs: the clusters (behind the last one: 0)
+    unsigned short cl[kMaxU];                    // runs: the clusters (behind an odd number of them the first one again)
     union {
         unsigned char map[kTR][kMaxU];           // [row][group]: place of the group in the row + 1, 0: not named by it
         unsigned short lists[2][kGroupMaxM];     // same: source rows by slot (0xffff: absent, and so are the slots behind the last group)
@@ -175,7 +175,11 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
             }
         }
         if (!__any_sync(kFull, twice)) {
-            if (lane == 0) rec.head = kRecRuns | (unsigned)U << 8;
+            if (lane == 0) {
+                rec.head = kRecRuns | (unsigned)U << 8;
+                // groups are taken in pairs: what is multiplied with zeros in place of one more must be the tile's own rows
+                if (U & 1) rec.cl[U] = rec.cl[0];
+            }
             __syncwarp();
             return;
         }

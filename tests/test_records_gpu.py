@@ -74,3 +74,22 @@ def test_clusters_far_apart(lib):
     f, da, dv = formula.forward_backward("av", d[2], d[3], idx, g_feat.double())
     for name, x, w in zip(("attn", "feat", "d_query", "d_key", "d_attn", "d_value"), got, (a, f, dq, dk, da, dv)):
         assert rel_err(x, w) <= TOL[torch.float32], name
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["float32", "bfloat16"])
+@pytest.mark.parametrize("n", [3136, 1001])
+def test_tokens_that_a_tile_does_not_name(lib, n, dtype):
+    """Values that are not finite stay with the tiles of 16 rows that name them; an odd number of clusters is padded with the
+    tile's own."""
+    from clusten import CLUSTENAVFunction, ops
+    idx = workloads.make_index("model", 1, n, 48, 620, DEV)
+    g = torch.Generator(device=DEV).manual_seed(621)
+    attn, v, q = (torch.randn(1, 2, n, w, generator=g, device=DEV).to(dtype) for w in (48, 32, 32))
+    v[:, :, :8] = float("nan")
+    named = torch.zeros(16 * ((n + 15) // 16), dtype=torch.bool, device=DEV)
+    named[:n] = (idx[0] < 8).any(1)
+    clean = ~named.view(-1, 16).any(1, keepdim=True).expand(-1, 16).reshape(-1)[:n]
+    assert clean.float().mean() > 0.5
+    assert torch.isfinite(CLUSTENAVFunction.apply(attn, v, idx)[:, :, clean]).all()
+    assert torch.isfinite(ops.local_attention_forward(q, q, v, idx)[:, :, clean]).all()
+    assert torch.isfinite(ops.local_attention_forward(q, v, q, idx)[:, :, clean]).all()
