@@ -422,8 +422,8 @@ fused_attention_kernel(const __grid_constant__ FusedParams p) {
             blank[e] += __shfl_xor_sync(kFull, blank[e], 1);
             blank[e] += __shfl_xor_sync(kFull, blank[e], 2);
             blank[e] *= kLog2e;
-            st.ref[e] = p.blank_k ? blank[e] : 0.f;
-            st.set[e] = p.blank_k != nullptr;
+            st.set[e] = p.blank_k && blank[e] > -INFINITY;   // (no reference: minus infinity, NaN)
+            st.ref[e] = st.set[e] ? blank[e] : 0.f;
             st.sum[e] = make_float2(0.f, 0.f);
         }
         float acc[2][2][4];

@@ -113,6 +113,23 @@ def test_dense_bias_at_the_end_of_a_buffer(lib, n, dtype):
     assert rel_err(got, _chain(q, k, v, idx, bias)) <= TOL[dtype]
 
 
+def test_blank_logits_that_are_not_finite(lib):
+    """A blank logit of minus infinity takes no part (2^-x of it is no reference for the others), one of NaN makes the row NaN."""
+    from clusten import ops
+    b, h, n, m, c = 1, 2, 200, 48, 32
+    idx = workloads.make_index("model", b, n, m, 430, DEV)
+    g = torch.Generator(device=DEV).manual_seed(431)
+    q, k, v = (torch.randn(b, h, n, c, generator=g, device=DEV) for _ in range(3))
+    q[..., 0], k[..., 0] = 1e20, 1e-20
+    blank_k, blank_v = torch.zeros(h, c, device=DEV), torch.randn(h, c, generator=g, device=DEV)
+    blank_k[0, 0] = -1e30                                    # 1e20 * -1e30: minus infinity in fp32
+    q[:, 1, :16, 1], blank_k[1, 1] = float("nan"), 1.0
+    got = ops.local_attention_forward(q, k, v, idx, blank_k=blank_k, blank_v=blank_v)
+    want = _chain(q[:, :1], k[:, :1], v[:, :1], idx, blank_k=blank_k[:1], blank_v=blank_v[:1])
+    assert rel_err(got[:, :1], want) <= TOL[torch.float32]
+    assert torch.isnan(got[:, 1, :16]).all() and torch.isfinite(got[:, 1, 16:]).all()
+
+
 def test_argument_checks(lib):
     p = 256
     call = lib.clusten_local_attention_forward
