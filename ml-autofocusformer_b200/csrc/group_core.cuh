@@ -557,10 +557,51 @@ template <typename T> __device__ __forceinline__ void store_rows8(const float (&
 template <typename T> __device__ __forceinline__ void store_set(const float (&d)[2][4], T* out, int rows, int lane) { store_rows8(d, out, kC, rows, lane); }
 __device__ __forceinline__ unsigned byte_of(unsigned w, int i) { return __byte_perm(w, 0u, 0x4440u + i); }
 
+// ---- copies to shared memory and operands from there (16-bit); addresses are 32-bit shared ones
+__device__ __forceinline__ void cp_async16_or_zero(unsigned dst, const void* src, bool there) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], unsigned a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x2_trans(unsigned (&r)[2], unsigned a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void stmatrix_x4_trans(unsigned a, unsigned r0, unsigned r1, unsigned r2, unsigned r3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+}
+__device__ __forceinline__ unsigned lds16(unsigned a) {
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned lds32(unsigned a) {
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint4 lds128(unsigned a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cp_async16_cg(unsigned dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+// Rows of 64 bytes in shared memory: the 16-byte piece c of row r lies at place c ^ (r / 2) % 4, so that neither 8 rows' pieces c (ldmatrix)
+// nor the four pieces of two rows (16-byte accesses) share a bank
+__device__ __forceinline__ unsigned row_piece(int r, int c) { return 64u * r + 16u * (c ^ ((r >> 1) & 3)); }
+// out^T accumulators (M tile mt: channels 16 mt + g, + 8; columns 2t, 2t + 1: rows) of 8 rows -> rows of 64 bytes at buf
+template <typename T> __device__ __forceinline__ void acc_to_rows(const float (&d)[2][4], unsigned buf, int lane) {
+    const T* e = nullptr;
+    stmatrix_x4_trans(buf + row_piece(lane & 7, lane >> 3), pack2(d[0][0], d[0][1], e), pack2(d[0][2], d[0][3], e), pack2(d[1][0], d[1][1], e), pack2(d[1][2], d[1][3], e));
+}
+
 // Heads per warp.  A warp that serves all heads reads its tile's record once; when the tiles alone leave the chip short
-// of warps (24 per SM), the heads are spread over several warps.
-inline void split_heads(long long tiles, int heads, int* parts, int* per_part) {
-    const long long want = (long long)sm_count() * 24;
+// of warps (`warps` per SM), the heads are spread over several warps.
+inline void split_heads(long long tiles, int heads, int* parts, int* per_part, int warps = 24) {
+    const long long want = (long long)sm_count() * warps;
     int per = heads;
     while (per > 1 && tiles * ((heads + per - 1) / per) < want) per = (per + 1) / 2;
     *per_part = per;

@@ -4,11 +4,11 @@
 //
 // A warp takes the 8 targets 8T .. 8T+7 of a batch element and some or all heads and forms
 // out^T[channel][target] = X^T[channel][row] * W[row][target] on the tensor cores (FP32 inputs as TF32 in three passes).
-// Lane (g, t) = (lane / 4, lane % 4) reads 4 channels of the rows whose products it feeds, and the weights of those rows for
-// target 8T + g: in an AutoFocusFormer table the 8 targets of a row that names the cluster are 8 neighbouring weights, so a
-// request covers 4 rows times 16 or 32 contiguous bytes, and rows that do not name it are not read at all.  Operands go
-// from L1 / L2 into registers; no shared memory, no de-duplication, no atomics, a fixed order of summation.
-//   16-bit: one m16n8k16 step is 16 "runs" entries or the 8 rows of two "lists" entries; fp32: two steps of 8.
+// 16-bit, whole clusters: scatter_runs16.  Else lane (g, t) = (lane / 4, lane % 4) reads 4 channels of the rows whose products it
+// feeds, and the weights of those rows for target 8T + g: in an AutoFocusFormer table the 8 targets of a row that names the cluster
+// are 8 neighbouring weights, so a request covers 4 rows times 16 or 32 contiguous bytes, and rows that do not name it are not read at
+// all.  Operands go from L1 / L2 into registers; no de-duplication, no atomics, a fixed order of summation.
+//   16-bit: one m16n8k16 step is the 8 rows of two "lists" entries; fp32: two steps of 8 rows.
 // Batch elements with the ordinary index (random tables) take the targets one after the other, 16 (8) entries per step.
 //
 // The reference adds every (row, slot, channel) term with atomicAdd (clusten/src/clustenqk_cuda_kernel.cu:117-127,
@@ -92,9 +92,124 @@ __device__ __forceinline__ void step_rows(float (&acc)[2][4], const T* const (&r
     }
 }
 
-template <typename T, bool M48, bool TAIL>
+// ----------------------------------------------------------------------------- whole clusters, 16-bit
+// A step is 16 entries of the tile's list.  Its 16 rows of X (64 bytes each) and the 16 x 8 weights travel to shared memory by
+// cp.async, kSDepth - 1 steps ahead and across the warp's heads, and come back as operands by ldmatrix.trans.  The entries
+// behind the last one (place 0) are filled with zeros without a look at memory.  Against rows and weights that went from L1 straight
+// into operand registers: b128 h2 n3136 bf16 121 -> 97 us, b32 h8 n1843 fp16 111 -> 63, b128 h8 n196 bf16 62 -> 34 (in the last two
+// one more walk over the padded cluster's list instead of one per padded slot).  Bound by the L1 (83 % busy): a row of X or of
+// weights is a line of its own.
+constexpr int kSDepth = 2;                        // (3: the same times with 20 % more shared memory; 4: b128 h2 n3136 bf16 120 us, for want of L1)
+template <bool SHIFT> struct RunsStage {
+    static constexpr int kW = 16 * 64;                       // 16 rows of X (row_piece)
+    static constexpr int kAt = kW + 16 * (SHIFT ? 32 : 16);  // weights; SHIFT (rows start anywhere): the two aligned pieces that cover them,
+    static constexpr int kBytes = kAt + (SHIFT ? 32 : 0);    // and at which byte of them the first one is
+    static constexpr int kWarp = kSDepth * kBytes + 8 * 64;  // and the output tile
+};
+
+// sm: the warp's RunsStage::kWarp bytes;  list, own: the tile's entries and its steps;  pad_list, pad: those of the padded cluster, whose
+// slots from `first_pad` on name token 0 (tile 0 only; else pad = 0);  w, x: of the first head;  out: the tile's rows there
+template <typename T, bool SHIFT, bool TAIL>
+__device__ __forceinline__ void scatter_runs16(unsigned char* sm, const unsigned* list, int own, const unsigned* pad_list, int pad, int first_pad,
+                                               int heads, const T* w, long long w_head, int w_row, const T* x, long long x_head, int x_row, T* out,
+                                               long long out_head, int rows, int lane) {
+    using S = RunsStage<SHIFT>;
+    const int g = lane >> 2, t = lane & 3;
+    const unsigned base = smem_u32(sm), obuf = base + kSDepth * S::kBytes;
+    const int per_head = pad + own;
+    // ---- copies: rows lane / 4 and 8 + lane / 4, piece lane % 4
+    const unsigned x_dst = base + row_piece(g, t);
+    const char* xi = reinterpret_cast<const char*>(x) + 16 * t;
+    const unsigned x_bytes = 2u * (unsigned)x_row;
+    const T* wi = w - 8;
+    int left = per_head * heads, step = 0;
+    unsigned next = left > 0 ? __ldg((pad > 0 ? pad_list : list) + (lane & 15)) : 0u;
+    unsigned stage = 0u;
+    auto issue = [&]() {
+        if (left > 0) {
+            const unsigned e = next;
+            const char* xh = xi;
+            const T* wh = wi;
+            --left;
+            if (++step == per_head) {
+                step = 0;
+                xi += 2 * x_head;
+                wi += w_head;
+            }
+            if (left > 0) next = __ldg((TAIL && step < pad ? pad_list + 16 * step : list + 16 * (step - pad)) + (lane & 15));
+            const unsigned e0 = __shfl_sync(kFull, e, g), e1 = __shfl_sync(kFull, e, 8 + g);
+            cp_async16_or_zero(x_dst + stage, xh + (unsigned long long)(e0 >> 8) * x_bytes, (e0 & 255u) != 0u);
+            cp_async16_or_zero(x_dst + stage + 512, xh + (unsigned long long)(e1 >> 8) * x_bytes, (e1 & 255u) != 0u);
+            if (SHIFT) {
+                const unsigned ew = __shfl_sync(kFull, e, lane >> 1);
+                const uintptr_t at = reinterpret_cast<uintptr_t>(wh + (unsigned long long)(ew >> 8) * (unsigned)w_row + 8 * (ew & 255u));
+                const unsigned off = (unsigned)at & 15u;
+                const bool there = (ew & 255u) != 0u && ((lane & 1) == 0 || off != 0u);
+                cp_async16_or_zero(base + stage + S::kW + 16 * lane, reinterpret_cast<const void*>((at & ~uintptr_t(15)) + 16 * (lane & 1)), there);
+                if ((lane & 1) == 0)
+                    asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(base + stage + S::kAt + lane), "h"((unsigned short)(16 * lane + off)) : "memory");
+            } else if (lane < 16) {
+                cp_async16_or_zero(base + stage + S::kW + 16 * lane, wh + (unsigned long long)(e >> 8) * (unsigned)w_row + 8 * (e & 255u), (e & 255u) != 0u);
+            }
+            stage = stage == (kSDepth - 1) * S::kBytes ? 0u : stage + S::kBytes;
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int d = 0; d < kSDepth - 1; ++d) issue();
+    // ---- products
+    const int r = (lane & 7) + 8 * (lane >> 4), c = (lane >> 3) & 1;
+    const unsigned a_at = base + row_piece(r, c), a_at2 = base + row_piece(r, c + 2);
+    unsigned now = 0u;
+    for (int h = 0; h < heads; ++h) {
+        float acc[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[0][i] = acc[1][i] = 0.f;
+        for (int s = 0; s < per_head; ++s) {
+            cp_async_wait<kSDepth - 2>();
+            __syncwarp();
+            issue();
+            unsigned a[2][4], bw[2];
+            ldmatrix_x4_trans(a[0], a_at + now);
+            ldmatrix_x4_trans(a[1], a_at2 + now);
+            if (SHIFT) {
+                const unsigned o0 = lds32(base + now + S::kAt + 4 * t), o1 = lds32(base + now + S::kAt + 16 + 4 * t);
+                const unsigned wb = base + now + S::kW + 2 * g;
+                bw[0] = lds16(wb + (o0 & 0xffffu)) | lds16(wb + (o0 >> 16)) << 16;
+                bw[1] = lds16(wb + (o1 & 0xffffu)) | lds16(wb + (o1 >> 16)) << 16;
+            } else {
+                ldmatrix_x2_trans(bw, base + now + S::kW + 16 * (lane & 15));
+            }
+            mma16(acc[0], a[0], bw, static_cast<const T*>(nullptr));
+            mma16(acc[1], a[1], bw, static_cast<const T*>(nullptr));
+            now = now == (kSDepth - 1) * S::kBytes ? 0u : now + S::kBytes;
+            if (TAIL && s == pad - 1) {
+                // the padded slots are all token 0: their columns -> column 0
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    float* d = &acc[i >> 2][i & 3];
+                    float sum = (2 * t >= first_pad ? d[0] : 0.f) + (2 * t + 1 >= first_pad ? d[1] : 0.f);
+                    sum += __shfl_xor_sync(kFull, sum, 1);
+                    sum += __shfl_xor_sync(kFull, sum, 2);
+                    d[0] = t == 0 ? sum : 0.f;
+                    d[1] = 0.f;
+                }
+            }
+        }
+        // acc: channels g, g + 8 (and 16, 24 more) of targets 2t, 2t + 1 -> rows of 64 bytes
+        __syncwarp();
+        acc_to_rows<T>(acc, obuf, lane);
+        __syncwarp();
+        if (g < rows) *reinterpret_cast<uint4*>(out + g * kC + 8 * t) = lds128(obuf + row_piece(g, t));
+        out += out_head;
+    }
+    cp_async_wait<0>();
+}
+
+template <typename T, bool M48, bool TAIL, bool SHIFT>
 __global__ void __launch_bounds__(32 * kSGWarps, 8)
 scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned task = blockIdx.x * kSGWarps + warp;
     if (task >= p.total) return;
@@ -116,13 +231,28 @@ scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
         start = __ldg(rowptr + tile);
         count = __ldg(seglen + tile);
     }
+    if constexpr (sizeof(T) == 2) {
+        if (mode == kBuildGroupRuns) {
+            int pad_start = 0, pad_count = 0;
+            if (TAIL && tile == 0) {
+                pad_start = __ldg(rowptr + (n >> 3));
+                pad_count = __ldg(seglen + (n >> 3));
+            }
+            const unsigned* list = reinterpret_cast<const unsigned*>(ents);
+            scatter_runs16<T, SHIFT, TAIL>(smem_raw + warp * RunsStage<SHIFT>::kWarp, list + start, count >> 4, list + pad_start, pad_count >> 4, n & 7, h1 - h0,
+                                           Wb + (long long)h0 * p.w_head, p.w_head, p.w_row,
+                                           static_cast<const T*>(p.X) + (long long)b * p.x_batch + (long long)h0 * p.x_head, p.x_head, p.x_row,
+                                           static_cast<T*>(p.out) + (((long long)b * p.heads + h0) * n + tile * 8) * kC, (long long)n * kC, n - tile * 8, lane);
+            return;
+        }
+    }
     for (int h = h0; h < h1; ++h) {
         const T* W = Wb + (long long)h * p.w_head;
         const T* X = Xb + (long long)h * p.x_head;
         float acc[2][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[0][i] = acc[1][i] = 0.f;
-        if (mode == kBuildGroupRuns) {
+        if (sizeof(T) == 4 && mode == kBuildGroupRuns) {
             // 16 rows a step, 4 per lane, the next step's entries on their way
             const T* Wg = W + g - 8;
             auto walk = [&](const uint4* list, int steps, const T* w0, bool live) {
@@ -229,10 +359,19 @@ scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
 
 template <typename T>
 int scatter_groups_t(const char* label, ScatterGroupsParams p, cudaStream_t s) {
-    auto kernel = p.n & 7 ? (p.m == 48 ? scatter_groups_kernel<T, true, true> : scatter_groups_kernel<T, false, true>)
-                          : (p.m == 48 ? scatter_groups_kernel<T, true, false> : scatter_groups_kernel<T, false, false>);
+    constexpr int kPer = 16 / (int)sizeof(T);
+    const bool shift = sizeof(T) == 2 && (reinterpret_cast<uintptr_t>(p.W) % 16 != 0 || p.w_row % kPer != 0 || p.w_batch % kPer != 0 || p.w_head % kPer != 0);
+    auto pick = [&](auto m48, auto tail) {
+        constexpr bool M48 = decltype(m48)::value, TAIL = decltype(tail)::value;
+        return shift ? scatter_groups_kernel<T, M48, TAIL, sizeof(T) == 2> : scatter_groups_kernel<T, M48, TAIL, false>;
+    };
+    auto kernel = p.n & 7 ? (p.m == 48 ? pick(std::true_type{}, std::true_type{}) : pick(std::false_type{}, std::true_type{}))
+                          : (p.m == 48 ? pick(std::true_type{}, std::false_type{}) : pick(std::false_type{}, std::false_type{}));
+    const int smem = sizeof(T) == 2 ? kSGWarps * (shift ? RunsStage<true>::kWarp : RunsStage<false>::kWarp) : 0;
+    const int fit = resident_ctas(reinterpret_cast<const void*>(kernel), 32 * kSGWarps, smem);
+    if (fit < 0) return fit;
     ScopedKernelTimer timer(label, s);
-    kernel<<<(p.total + kSGWarps - 1) / kSGWarps, 32 * kSGWarps, 0, s>>>(p);
+    kernel<<<(p.total + kSGWarps - 1) / kSGWarps, 32 * kSGWarps, smem, s>>>(p);
     note_launch();
     return check_launch();
 }
@@ -249,7 +388,8 @@ int launch_scatter_groups(const char* label, int dtype, const void* W, const voi
     p.heads = h;  p.n = n;  p.m = m;
     const long long tiles = (long long)b * inv.ntiles;
     if (tiles * h > 0x7fffffffLL) return CLUSTEN_ERR_SHAPE;
-    split_heads(tiles, h, &p.parts, &p.per_part);
+    // 16-bit warps have little to read before the first head: more of them (b32 h8 n1843 fp16 63 us, 70 with 24 per SM; b128 h8 n196 bf16 33, 37)
+    split_heads(tiles, h, &p.parts, &p.per_part, dtype == CLUSTEN_F32 ? 24 : 64);
     p.total = (unsigned)(tiles * p.parts);
     while ((1ull << p.m_shift) < (unsigned)m) ++p.m_shift;
     p.m_magic = (unsigned)(((1ull << 32) * ((1ull << p.m_shift) - (unsigned)m)) / (unsigned)m + 1);
