@@ -4,11 +4,11 @@
 //
 // A warp takes the 8 targets 8T .. 8T+7 of a batch element and some or all heads and forms
 // out^T[channel][target] = X^T[channel][row] * W[row][target] on the tensor cores (FP32 inputs as TF32 in three passes).
-// 16-bit, whole clusters: scatter_runs16.  Else lane (g, t) = (lane / 4, lane % 4) reads 4 channels of the rows whose products it
+// 16-bit, whole clusters and lists: scatter_runs16, scatter_lists16.  Else lane (g, t) = (lane / 4, lane % 4) reads 4 channels of the rows whose products it
 // feeds, and the weights of those rows for target 8T + g: in an AutoFocusFormer table the 8 targets of a row that names the cluster
 // are 8 neighbouring weights, so a request covers 4 rows times 16 or 32 contiguous bytes, and rows that do not name it are not read at
 // all.  Operands go from L1 / L2 into registers; no de-duplication, no atomics, a fixed order of summation.
-//   16-bit: one m16n8k16 step is the 8 rows of two "lists" entries; fp32: two steps of 8 rows.
+//   16-bit: one m16n8k16 step is 16 entries; fp32: two steps of 8 rows.
 // Batch elements with the ordinary index (random tables) take the targets one after the other, 16 (8) entries per step.
 //
 // The reference adds every (row, slot, channel) term with atomicAdd (clusten/src/clustenqk_cuda_kernel.cu:117-127,
@@ -104,8 +104,17 @@ template <bool SHIFT> struct RunsStage {
     static constexpr int kW = 16 * 64;                       // 16 rows of X (row_piece)
     static constexpr int kAt = kW + 16 * (SHIFT ? 32 : 16);  // weights; SHIFT (rows start anywhere): the two aligned pieces that cover them,
     static constexpr int kBytes = kAt + (SHIFT ? 32 : 0);    // and at which byte of them the first one is
-    static constexpr int kWarp = kSDepth * kBytes + 8 * 64;  // and the output tile
+    static constexpr int kWarp = kSDepth * kBytes;
 };
+
+// acc: channels g, g + 8 (and 16, 24 more) of targets 2t, 2t + 1 -> the tile's rows, by way of the stage at buf, whose operands have been read
+template <typename T> __device__ __forceinline__ void store_targets(const float (&acc)[2][4], unsigned buf, T* out, int rows, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    __syncwarp();
+    acc_to_rows<T>(acc, buf, lane);
+    __syncwarp();
+    if (g < rows) *reinterpret_cast<uint4*>(out + g * kC + 8 * t) = lds128(buf + row_piece(g, t));
+}
 
 // sm: the warp's RunsStage::kWarp bytes;  list, own: the tile's entries and its steps;  pad_list, pad: those of the padded cluster, whose
 // slots from `first_pad` on name token 0 (tile 0 only; else pad = 0);  w, x: of the first head;  out: the tile's rows there
@@ -115,7 +124,7 @@ __device__ __forceinline__ void scatter_runs16(unsigned char* sm, const unsigned
                                                long long out_head, int rows, int lane) {
     using S = RunsStage<SHIFT>;
     const int g = lane >> 2, t = lane & 3;
-    const unsigned base = smem_u32(sm), obuf = base + kSDepth * S::kBytes;
+    const unsigned base = smem_u32(sm);
     const int per_head = pad + own;
     // ---- copies: rows lane / 4 and 8 + lane / 4, piece lane % 4
     const unsigned x_dst = base + row_piece(g, t);
@@ -196,11 +205,83 @@ __device__ __forceinline__ void scatter_runs16(unsigned char* sm, const unsigned
                 }
             }
         }
-        // acc: channels g, g + 8 (and 16, 24 more) of targets 2t, 2t + 1 -> rows of 64 bytes
-        __syncwarp();
-        acc_to_rows<T>(acc, obuf, lane);
-        __syncwarp();
-        if (g < rows) *reinterpret_cast<uint4*>(out + g * kC + 8 * t) = lds128(obuf + row_piece(g, t));
+        store_targets<T>(acc, base + (now == 0u ? (kSDepth - 1) * S::kBytes : now - S::kBytes), out, rows, lane);
+        out += out_head;
+    }
+    cp_async_wait<0>();
+}
+
+// Lists, 16-bit: a step is two entries, 8 + 8 rows; the rows travel as above, the weights -- one slot for each target, wherever it lies in the row --
+// one step ahead into the registers of the lanes that feed them.  Training passes over tables shared by a cluster, d_query and d_key / d_attn and
+// d_value: b128 h2 n3136 bf16 216, 232 -> 200, 205 us, b64 h8 n784 m24 98, 97 -> 76, 82.  ents: the tile's entries, `count` of them
+template <typename T, int STAGE>
+__device__ __forceinline__ void scatter_lists16(unsigned char* sm, const uint4* ents, int count, int heads, const T* w, long long w_head, int w_row, const T* x,
+                                                long long x_head, int x_row, T* out, long long out_head, int n, int rows, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    const unsigned base = smem_u32(sm), x_dst = base + row_piece(g, t), x_bytes = 2u * (unsigned)x_row;
+    const char* xi = reinterpret_cast<const char*>(x) + 16 * t;
+    const T* wi = w;
+    const int per_head = (count + 1) >> 1;
+    int left = per_head * heads, step = 0;
+    const uint4 none = make_uint4((unsigned)n, 0xffffffffu, 0xffffffffu, 0u);
+    uint4 e[2] = {none, none};
+    auto load = [&](int s) {
+        e[0] = __ldg(ents + 2 * s);
+        e[1] = 2 * s + 1 < count ? __ldg(ents + 2 * s + 1) : none;
+    };
+    if (left > 0) load(0);
+    unsigned stage = 0u, coming[2] = {0u, 0u};
+    auto issue = [&]() {
+        if (left > 0) {
+            const char* xh = xi;
+            const T* wh = wi;
+            const uint4 now[2] = {e[0], e[1]};
+            --left;
+            if (++step == per_head) {
+                step = 0;
+                xi += 2 * x_head;
+                wi += w_head;
+            }
+            if (left > 0) load(step);
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+                const unsigned row = now[z].x + g;
+                cp_async16_or_zero(x_dst + stage + 512 * z, xh + (unsigned long long)(row < (unsigned)n ? row : 0u) * x_bytes, row < (unsigned)n);
+                const unsigned j = ((g & 4 ? now[z].z : now[z].y) >> (8 * (g & 3))) & 0xffu;
+                unsigned v[2] = {0u, 0u};
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const unsigned r = now[z].x + 2 * t + i;
+                    if (j != 0xffu && r < (unsigned)n) v[i] = __ldg(reinterpret_cast<const unsigned short*>(wh + (unsigned long long)r * (unsigned)w_row + j));
+                }
+                coming[z] = v[0] | v[1] << 16;
+            }
+            stage = stage == (kSDepth - 1) * STAGE ? 0u : stage + STAGE;
+        }
+        cp_async_commit();
+    };
+    static_assert(kSDepth == 2, "the weights are one step ahead");
+    issue();
+    const int r = (lane & 7) + 8 * (lane >> 4), c = (lane >> 3) & 1;
+    const unsigned a_at = base + row_piece(r, c), a_at2 = base + row_piece(r, c + 2);
+    unsigned now = 0u;
+    for (int h = 0; h < heads; ++h) {
+        float acc[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[0][i] = acc[1][i] = 0.f;
+        for (int s = 0; s < per_head; ++s) {
+            const unsigned bw[2] = {coming[0], coming[1]};
+            cp_async_wait<0>();
+            __syncwarp();
+            issue();
+            unsigned a[2][4];
+            ldmatrix_x4_trans(a[0], a_at + now);
+            ldmatrix_x4_trans(a[1], a_at2 + now);
+            mma16(acc[0], a[0], bw, static_cast<const T*>(nullptr));
+            mma16(acc[1], a[1], bw, static_cast<const T*>(nullptr));
+            now = STAGE - now;
+        }
+        store_targets<T>(acc, base + STAGE - now, out, rows, lane);
         out += out_head;
     }
     cp_async_wait<0>();
@@ -232,6 +313,10 @@ scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
         count = __ldg(seglen + tile);
     }
     if constexpr (sizeof(T) == 2) {
+        unsigned char* sm = smem_raw + warp * RunsStage<SHIFT>::kWarp;
+        const T* W0 = Wb + (long long)h0 * p.w_head;
+        const T* X0 = static_cast<const T*>(p.X) + (long long)b * p.x_batch + (long long)h0 * p.x_head;
+        T* out0 = static_cast<T*>(p.out) + (((long long)b * p.heads + h0) * n + tile * 8) * kC;
         if (mode == kBuildGroupRuns) {
             int pad_start = 0, pad_count = 0;
             if (TAIL && tile == 0) {
@@ -239,10 +324,12 @@ scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
                 pad_count = __ldg(seglen + (n >> 3));
             }
             const unsigned* list = reinterpret_cast<const unsigned*>(ents);
-            scatter_runs16<T, SHIFT, TAIL>(smem_raw + warp * RunsStage<SHIFT>::kWarp, list + start, count >> 4, list + pad_start, pad_count >> 4, n & 7, h1 - h0,
-                                           Wb + (long long)h0 * p.w_head, p.w_head, p.w_row,
-                                           static_cast<const T*>(p.X) + (long long)b * p.x_batch + (long long)h0 * p.x_head, p.x_head, p.x_row,
-                                           static_cast<T*>(p.out) + (((long long)b * p.heads + h0) * n + tile * 8) * kC, (long long)n * kC, n - tile * 8, lane);
+            scatter_runs16<T, SHIFT, TAIL>(sm, list + start, count >> 4, list + pad_start, pad_count >> 4, n & 7, h1 - h0, W0, p.w_head, p.w_row, X0, p.x_head, p.x_row, out0,
+                                           (long long)n * kC, n - tile * 8, lane);
+            return;
+        }
+        if (mode == kBuildGroupLists) {
+            scatter_lists16<T, RunsStage<SHIFT>::kBytes>(sm, ents + start, count, h1 - h0, W0, p.w_head, p.w_row, X0, p.x_head, p.x_row, out0, (long long)n * kC, n, n - tile * 8, lane);
             return;
         }
     }
@@ -277,7 +364,7 @@ scatter_groups_kernel(const __grid_constant__ ScatterGroupsParams p) {
                 const int last = n >> 3, s1 = __ldg(rowptr + last), c1 = __ldg(seglen + last);
                 for (int q = n & 7; q < 8; ++q) walk(ents + (s1 >> 2), c1 >> 4, Wg + q, g == 0);
             }
-        } else if (mode == kBuildGroupLists) {
+        } else if (sizeof(T) == 4 && mode == kBuildGroupLists) {
             // two entries of 8 rows per step: rows t and t + 4 of each
             uint4 e[2];
             auto load = [&](int k) {
