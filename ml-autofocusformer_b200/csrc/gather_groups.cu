@@ -16,6 +16,7 @@
 //         are laid out by row in shared memory (those of rows that do not name the group in front of them, where nobody
 //         looks) and leave as contiguous 16-byte pieces.
 //
+// 16-bit tiles of whole clusters share their rows with the three next ones (blocks of 64 rows, below).
 // FP32 inputs are multiplied as TF32 in three passes (tile_core.cuh), FP16 / BF16 inputs with m16n8k16.
 // The reference gives each output element a thread that re-gathers its neighbour rows from L2
 // (clusten/src/clustenav_cuda_kernel.cu:18-50, clustenqk_cuda_kernel.cu:18-49).
@@ -407,14 +408,14 @@ __device__ __forceinline__ void store_rows(const T* tile, T* __restrict__ out, i
 // MODE 0: sum, 1: dot;  RT: groups per row known at compile time (6: m = 48, every AutoFocusFormer stage) or 0;
 // SHIFT: the rows of the weights (sum) or scores (dot, LinearRows) do not start on 16-byte boundaries;  PLAN: the records are there;
 // TAIL: the last cluster is padded
-// CTAs per SM, measured for b128 h2 n3136 (and b32 h8 n1843).  dot: fp32 over records 7 (0.115 ms a call, 0.130 with 5), 5 where the
-// records are made here (b4 h2 n9216 22 us, 24 with 6); 16-bit 4, without spills (0.069 (0.056) ms, 0.079 (0.069) with 6).
-// sum: fp32 over records 5, 6 where they are made here (shared tables 134 us, 138 with 5; b128 h8 n196 45, 50 with 5), 16-bit 7
-// (0.086 (0.068) ms, 0.089 (0.083) with 6).
+// CTAs per SM, measured for b128 h2 n3136.  dot: fp32 over records 7 (0.115 ms a call, 0.130 with 5), 5 where the records are made here
+// (b4 h2 n9216 22 us, 24 with 6); 16-bit 4, without spills (b128 h8 n196 22.8 us, 28.3 with 6).  sum: fp32 over records 5, 6 where they are
+// made here (shared tables 134 us, 138 with 5; b128 h8 n196 45, 50 with 5), 16-bit 7.
 template <typename T, int MODE, bool PLAN> constexpr int gather_ctas() {
     if (MODE == 1) return sizeof(T) == 4 ? (PLAN ? 7 : 5) : 4;
     return sizeof(T) == 4 ? (PLAN ? 5 : 6) : 7;
 }
+constexpr int kBlockCtas = 6;                    // blocks (below): dot 66 us, sum 72 (5: 68, 72; 7: 62, 76; tables shared by a cluster 92, 97, 110)
 template <typename T, int MODE, int RT, bool SHIFT, bool PLAN, bool TAIL>
 __global__ void __launch_bounds__(32 * kGWarps, (gather_ctas<T, MODE, PLAN>()))
 gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
@@ -575,34 +576,370 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
     }
 }
 
+// ----------------------------------------------------------------------------- blocks of 64 rows, 16-bit
+// A CTA's four tiles are consecutive.  When all of them have whole clusters, the distinct ones among them -- 25 where the tiles by themselves
+// have 4 x 13 -- go to shared memory once per head, and the products read them there (sum: ldmatrix.trans, dot: 16-byte loads).  Against
+// tiles that read their own rows from L1 / L2, over records: b128 h2 n3136 bf16 dot 74 -> 66 us, sum 90 -> 72, b32 h8 n1843 fp16 60 -> 45,
+// 73 -> 50.  What is left is waiting: with its clusters on the way a block has nothing else to do, and six of them share an SM
+// (without the products the same blocks take 50 of the 66 us; the bytes that DRAM has to move, 37).
+constexpr int kBlockClusters = 40;               // with more of them (at most 35 in AutoFocusFormer's tables) each tile reads its own
+constexpr int kBlockBytes = kBlockClusters * 512;
+
+// Scores of a tile, 16 rows of 6 pieces of 8.  The pitch is an odd number of pieces, so that 8 rows' pieces of one place lie in different
+// banks.  Behind them 8 pieces for the scores that nobody names.
+constexpr int kBlockR = kMmax / 8;
+constexpr int kScorePitch = 16 * (kBlockR + 1), kScoreNone = kTR * kScorePitch, kScoreBytes = kScoreNone + 8 * 16;
+// One head, whole clusters.  xs: the block's rows (sm.rec.cl: places of the clusters there);  w, at, map: as for sum_head
+template <typename T, bool SHIFT, int SET>
+__device__ __forceinline__ void sum_runs(unsigned xs, const T* w, const PairAt (&at)[2], const unsigned char* map, const GroupSmem& sm, int U, int lane,
+                                         float (&acc)[2][2][4]) {
+    // rows of the operand: slots lane % 8 of group u (lanes 0-15) and u + 1, piece (lane / 8) % 2 and that + 2
+    const unsigned a0 = xs + row_piece(lane & 7, (lane >> 3) & 1), a1 = xs + row_piece(lane & 7, ((lane >> 3) & 1) + 2);
+    const unsigned short* cl = sm.rec.cl + (lane >> 4);
+#pragma unroll 1
+    for (int u0 = 0; u0 < U; u0 += 4) {
+        unsigned rm[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) rm[e] = *reinterpret_cast<const unsigned*>(map + 8 * e * kMaxU + u0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (h == 1 && u0 + 2 >= U) break;
+            const unsigned at_x = 512u * cl[u0 + 2 * h];
+            unsigned a[2][4];
+            ldmatrix_x4_trans(a[0], a0 + at_x);
+            ldmatrix_x4_trans(a[1], a1 + at_x);
+            auto weights = [&](int e, int i) -> unsigned {
+                const unsigned place = byte_of(rm[e], 2 * h + i);
+                const T* p = w + e * SET + 64 * place;
+                if (!SHIFT) return *reinterpret_cast<const unsigned*>(p);
+                const unsigned q = __funnelshift_r(*reinterpret_cast<const unsigned*>(p + at[e].first), *reinterpret_cast<const unsigned*>(p + at[e].second), at[e].bits);
+                return place == 0u ? 0u : q;
+            };
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const unsigned b[2] = {weights(e, 0), weights(e, 1)};
+                mma16(acc[e][0], a[0], b, static_cast<const T*>(nullptr));
+                mma16(acc[e][1], a[1], b, static_cast<const T*>(nullptr));
+            }
+        }
+    }
+}
+// q: rows g, g + 8, channels 8t .. 8t+7.  A record's places are row addresses for stmatrix: one instruction leaves the scores of both sets of rows
+// for two groups; a lane has row lane % 16 and the groups u + lane / 16
+template <typename T>
+__device__ __forceinline__ void dot_runs(const uint4 (&q)[2], unsigned xs, unsigned tile, const GroupSmem& sm, int U, int lane) {
+    const unsigned a0[4] = {q[0].x, q[1].x, q[0].y, q[1].y}, a1[4] = {q[0].z, q[1].z, q[0].w, q[1].w};
+    const T* type = nullptr;
+    const unsigned row = tile + (lane & 15) * kScorePitch - 16, none = tile + kScoreNone + 16 * (lane & 7);
+    const unsigned char* map = sm.rec.map[lane & 15];
+    xs += row_piece(lane >> 2, lane & 3);
+#pragma unroll 1
+    for (int u0 = 0; u0 < U; u0 += 4) {
+        const uint2 cl = *reinterpret_cast<const uint2*>(sm.rec.cl + u0);
+        const unsigned places = *reinterpret_cast<const unsigned*>(map + u0) >> (8 * (lane >> 4));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (h == 1 && u0 + 2 >= U) break;
+            const unsigned cc = h ? cl.y : cl.x, place = byte_of(places, 2 * h);
+            const uint4 k[2] = {lds128(xs + 512u * (cc & 0xffffu)), lds128(xs + 512u * (cc >> 16))};
+            float d[2][4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const unsigned b0[2] = {k[i].x, k[i].y}, b1[2] = {k[i].z, k[i].w};
+                mma16_first(d[i], a0, b0, type);
+                mma16(d[i], a1, b1, type);
+            }
+            stmatrix_x4(place ? row + 16 * place : none, pack2(d[0][0], d[0][1], type), pack2(d[0][2], d[0][3], type), pack2(d[1][0], d[1][1], type),
+                        pack2(d[1][2], d[1][3], type));
+        }
+    }
+}
+
+// A tile by itself, 16-bit, its record unpacked (the weights of the first head are on their way): as in gather_groups_kernel
+template <typename T, int MODE, bool SHIFT, bool TAIL>
+__device__ __forceinline__ void gather_tile(const GatherGroupsParams& p, GroupSmem& sm, T* tile, const T* A, const T* X, const int64_t* src, int b, int i0, int rows,
+                                            int h0, int h1, int lane) {
+    using Tile = RowTile<T, kBlockR, SHIFT>;
+    constexpr int m = kMmax;
+    const int n = p.n;
+    const int g = lane >> 2, t = lane & 3;
+    const unsigned head = sm.rec.head;
+    const unsigned kind = head & 0xffu;
+    const bool holes = (head >> 16 & (MODE == 1 ? 1u : 3u)) != 0u;
+    const int U0 = (head >> 8) & 0xffu;
+    auto at_row = [&](const T* x, int row) { return reinterpret_cast<const T*>(reinterpret_cast<const char*>(x) + (unsigned long long)row * p.x_row); };
+    for (int h = h0; h < h1; ++h) {
+        const long long bh = (long long)b * p.heads + h;
+        const T* Ah = A + (long long)h * p.a_head;
+        const T* Xh = X + (long long)h * p.x_head;
+        if constexpr (MODE == 0) {
+            if (h > h0) {                                    // (the first head's weights were requested above)
+                __syncwarp();
+                stage_rows<T, kBlockR, SHIFT>(Ah, p.a_row, rows, m, kBlockR, tile, lane);
+            }
+            const T* w = tile + g * 8 + (SHIFT ? 0 : 2 * t);
+            T* o = static_cast<T*>(p.out) + (bh * n + i0 + 2 * t) * kC + 4 * g;
+            if (kind == kRecRuns) {
+                float acc[2][2][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[0][0][i] = acc[0][1][i] = acc[1][0][i] = acc[1][1][i] = 0.f;
+                PairAt at[2] = {};
+                if (SHIFT) {
+                    at[0] = pair_at(Ah + (long long)g * p.a_row, t);
+                    at[1] = pair_at(Ah + (long long)(g + 8) * p.a_row, t);
+                }
+                sum_head<Pick<true, false, TAIL>, T, SHIFT, 2, Tile::kSet>(at_row(Xh, 2 * t), p.x_row, w, at, sm.rec.map[g], sm, sm.tok, U0, p.pad_cl, n, t, acc);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (8 * e + 2 * t < rows) st4(o + 8 * e * kC, acc_channels(acc[e], 0));
+                    if (8 * e + 2 * t + 1 < rows) st4(o + (8 * e + 1) * kC, acc_channels(acc[e], 1));
+                }
+            } else {
+                for (int e = 0; 8 * e < rows; ++e) {
+                    float acc[1][2][4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[0][0][i] = acc[0][1][i] = 0.f;
+                    PairAt at[1] = {};
+                    if (SHIFT) at[0] = pair_at(Ah + (long long)(g + 8 * e) * p.a_row, t);
+                    const T* we = w + e * Tile::kSet;
+                    const unsigned char* map = sm.rec.map[g + 8 * e];
+                    if (kind == kRecSame) {
+                        const unsigned short* tok = sm.tok + e * kGroupMaxM;
+                        if (holes) sum_head<Pick<false, true>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
+                        else sum_head<Pick<false, false>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
+                    } else {
+                        for (int first = 8 * e, U; first < min(rows, 8 * e + 8);) {
+                            first += load_piece<kBlockR>(src, first, rows, m, n, p.wide_idx != 0, sm, lane, &U);
+                            sum_head<Pick<false, true>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, sm.tok, U, -1, n, t, acc);
+                        }
+                    }
+                    if (8 * e + 2 * t < rows) st4(o + 8 * e * kC, acc_channels(acc[0], 0));
+                    if (8 * e + 2 * t + 1 < rows) st4(o + (8 * e + 1) * kC, acc_channels(acc[0], 1));
+                }
+            }
+        } else {
+            auto load_row = [&](uint4& q, int row) {
+                q = make_uint4(0u, 0u, 0u, 0u);
+                if (row < rows) q = __ldg(reinterpret_cast<const uint4*>(Ah + (long long)row * p.a_row + 8 * t));
+            };
+            __syncwarp();                                    // the tile is free again
+            auto out_rows = [&]() { return static_cast<T*>(p.out) + (bh * n + i0) * m; };
+            const LinearRows lin = {0, 0};
+            T* at0 = tile + g * 8 + 2 * t;
+            if (kind == kRecRuns) {
+                uint4 q[2];
+                load_row(q[0], g);
+                load_row(q[1], g + 8);
+                dot_head16<Pick<true, false, TAIL>, T, 2, Tile::kSet, false>(q, at_row(Xh, g), p.x_row, at0, sm.rec.map[g], sm, sm.tok, U0, p.pad_cl, n, g, lin);
+            } else {
+                for (int e = 0; 8 * e < rows; ++e) {
+                    uint4 q[1];
+                    load_row(q[0], 8 * e + g);
+                    auto one = [&](auto pick, const unsigned short* tok, int U) {
+                        dot_head16<decltype(pick), T, 1, Tile::kSet, false>(q, Xh, p.x_row, at0 + e * Tile::kSet, sm.rec.map[8 * e + g], sm, tok, U, -1, n, g, lin);
+                    };
+                    if (kind == kRecSame) {
+                        if (holes) one(Pick<false, true>{}, sm.tok + e * kGroupMaxM, U0);
+                        else one(Pick<false, false>{}, sm.tok + e * kGroupMaxM, U0);
+                    } else {
+                        for (int first = 8 * e, U; first < min(rows, 8 * e + 8);) {
+                            first += load_piece<kBlockR>(src, first, rows, m, n, p.wide_idx != 0, sm, lane, &U);
+                            one(Pick<false, true>{}, sm.tok, U);
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+            store_rows<T, kBlockR, false>(tile, out_rows(), rows, m, kBlockR, lane);
+        }
+    }
+}
+
+template <typename T, int MODE, bool SHIFT, bool TAIL>
+__global__ void __launch_bounds__(32 * kGWarps, kBlockCtas)
+gather_blocks_kernel(const __grid_constant__ GatherGroupsParams p) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned short block_cl[kBlockClusters];
+    __shared__ int block_count;
+    using Tile = RowTile<T, kBlockR, SHIFT>;
+    constexpr int kTile = MODE == 1 ? kScoreBytes : Tile::kBytes;
+    static_assert(kTile >= Tile::kBytes, "a tile by itself has its place");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char* base = smem_raw + warp * (int)(sizeof(GroupSmem) + kTile);
+    unsigned char* xbuf = smem_raw + kGWarps * (int)(sizeof(GroupSmem) + kTile);
+    GroupSmem& sm = *reinterpret_cast<GroupSmem*>(base);
+    T* tile = reinterpret_cast<T*>(base + sizeof(GroupSmem));
+    const unsigned blocks = (unsigned)(p.tiles + kGWarps - 1) / kGWarps, bb = blockIdx.x / (unsigned)p.parts;
+    const int part = (int)(blockIdx.x - bb * (unsigned)p.parts);
+    const int b = (int)(bb / blocks);
+    const int ti = (int)(bb - (unsigned)b * blocks) * kGWarps + warp;
+    const bool live = ti < p.tiles;
+    const int i0 = ti * kTR;
+    constexpr int m = kMmax;
+    const int n = p.n;
+    const int rows = live ? min(kTR, n - i0) : 0;
+    const int g = lane >> 2, t = lane & 3;
+    const int h0 = part * p.per_part, h1 = min(p.heads, h0 + p.per_part);
+    const T* A = static_cast<const T*>(p.A) + (long long)b * p.a_batch + (long long)i0 * p.a_row;
+    const int64_t* src = p.idx + ((long long)b * n + i0) * m;
+    const unsigned tile_s = smem_u32(tile);
+    if (live) {
+        reinterpret_cast<uint4*>(&sm.rec)[lane] = __ldg(reinterpret_cast<const uint4*>(p.plan + (long long)b * p.tiles + ti) + lane);
+        __syncwarp();
+        if (MODE == 0) {
+            if (!SHIFT) {                                    // the zeros of place 0
+                for (int z = lane; z < 2 * Tile::kPlace * (int)sizeof(T) / 16; z += 32) {
+                    constexpr int kPer = 16 / (int)sizeof(T);
+                    const int e = z / (Tile::kPlace / kPer), c = z % (Tile::kPlace / kPer);
+                    *reinterpret_cast<uint4*>(tile + e * Tile::kSet + c * kPer) = make_uint4(0u, 0u, 0u, 0u);
+                }
+            }
+            stage_rows<T, kBlockR, SHIFT>(A + (long long)h0 * p.a_head, p.a_row, rows, m, kBlockR, tile, lane);
+        }
+    }
+    if (__syncthreads_and(!live || (sm.rec.head & 0xffu) == kRecRuns)) {
+        // ---- the distinct clusters of the block: a bit each, their places by population count
+        unsigned* bits = reinterpret_cast<unsigned*>(xbuf);
+        unsigned short* before = reinterpret_cast<unsigned short*>(xbuf + 1024);
+        const int words = (n + 255) >> 8;                    // (at most 254)
+        for (int z = threadIdx.x; z < words; z += 32 * kGWarps) bits[z] = 0u;
+        __syncthreads();
+        const int U = live ? (int)(sm.rec.head >> 8 & 0xffu) : 0;
+        const unsigned cl = lane < U ? sm.rec.cl[lane] : 0u;
+        if (lane < U) atomicOr(&bits[cl >> 5], 1u << (cl & 31u));
+        __syncthreads();
+        if (warp == 0) {
+            int run = 0;
+            for (int z = 0; z < words; z += 32) {
+                const int v = z + lane < words ? __popc(bits[z + lane]) : 0;
+                int incl = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                if (z + lane < words) before[z + lane] = (unsigned short)(run + incl - v);
+                run += __shfl_sync(kFull, incl, 31);
+            }
+            if (lane == 0) block_count = run;
+        }
+        __syncthreads();
+        const int total = block_count;
+        if (total <= kBlockClusters) {
+            const unsigned place = before[cl >> 5] + __popc(bits[cl >> 5] & ((1u << (cl & 31u)) - 1u));
+            const unsigned place0 = __shfl_sync(kFull, place, 0);
+            if (lane < U) {
+                sm.rec.cl[lane] = (unsigned short)place;
+                block_cl[place] = (unsigned short)cl;
+            } else if (lane == U && (U & 1)) {
+                sm.rec.cl[U] = (unsigned short)place0;
+            }
+            const unsigned xs = smem_u32(xbuf), x_dst = xs + 512u * warp + row_piece(g, t);
+            const char* xh = static_cast<const char*>(p.X) + 2 * ((long long)b * p.x_batch + (long long)h0 * p.x_head) + (unsigned long long)g * p.x_row + 16 * t;
+            const T* Ah = A + (long long)h0 * p.a_head;
+            long long bh = (long long)b * p.heads + h0;
+            for (int h = h0; h < h1; ++h, xh += 2 * p.x_head, Ah += p.a_head, ++bh) {
+                __syncthreads();                             // the clusters of the head before, or the bits, are done with
+                unsigned dst = x_dst;
+#pragma unroll 2
+                for (int u = warp; u < total; u += kGWarps, dst += 512u * kGWarps) {
+                    const unsigned first = 8u * block_cl[u];
+                    const char* from = xh + (unsigned long long)first * p.x_row;
+                    if (TAIL && first + g >= (unsigned)n) from = xh - (unsigned long long)g * p.x_row;      // slots behind the last token: token 0
+                    cp_async16_cg(dst, from);
+                }
+                if (MODE == 0 && h > h0 && live) stage_rows<T, kBlockR, SHIFT>(Ah, p.a_row, rows, m, kBlockR, tile, lane);
+                cp_async_commit();
+                if constexpr (MODE == 0) {
+                    cp_async_wait<0>();
+                    __syncthreads();
+                    if (!live) continue;
+                    float acc[2][2][4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[0][0][i] = acc[0][1][i] = acc[1][0][i] = acc[1][1][i] = 0.f;
+                    PairAt at[2] = {};
+                    if (SHIFT) {
+                        at[0] = pair_at(Ah + (long long)g * p.a_row, t);
+                        at[1] = pair_at(Ah + (long long)(g + 8) * p.a_row, t);
+                    }
+                    sum_runs<T, SHIFT, Tile::kSet>(xs, tile + g * 8 + (SHIFT ? 0 : 2 * t), at, sm.rec.map[g], sm, U, lane, acc);
+                    const unsigned buf = smem_u32(sm.tok);
+                    T* o = static_cast<T*>(p.out) + (bh * n + i0 + g) * kC + 8 * t;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        __syncwarp();
+                        acc_to_rows<T>(acc[e], buf, lane);
+                        __syncwarp();
+                        if (8 * e + g < rows) *reinterpret_cast<uint4*>(o + 8 * e * kC) = lds128(buf + row_piece(g, t));
+                    }
+                } else {
+                    uint4 q[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        q[e] = make_uint4(0u, 0u, 0u, 0u);
+                        if (8 * e + g < rows) q[e] = __ldg(reinterpret_cast<const uint4*>(Ah + (long long)(8 * e + g) * p.a_row + 8 * t));
+                    }
+                    cp_async_wait<0>();
+                    __syncthreads();
+                    if (!live) continue;
+                    dot_runs<T>(q, xs, tile_s, sm, U, lane);
+                    __syncwarp();
+                    T* o = static_cast<T*>(p.out) + (bh * n + i0) * m;
+#pragma unroll
+                    for (int k = 0; k < kBlockR / 2; ++k) {
+                        const int z = lane + 32 * k, row = z / kBlockR, j = z - row * kBlockR;
+                        if (row < rows) *reinterpret_cast<uint4*>(o + 8 * z) = lds128(tile_s + row * kScorePitch + 16 * j);
+                    }
+                }
+            }
+            return;
+        }
+    }
+    if (!live) return;
+    unpack_record<MODE == 1>(sm, rows, lane);
+    gather_tile<T, MODE, SHIFT, TAIL>(p, sm, tile, A, static_cast<const T*>(p.X) + (long long)b * p.x_batch + (MODE == 0 ? 4 * g : 8 * t), src, b, i0, rows,
+                                          h0, h1, lane);
+}
+
 template <typename T, int MODE>
 int gather_groups_t(const char* label, GatherGroupsParams p, int b, cudaStream_t s) {
     p.tiles = group_tiles(p.n);
     p.R = (p.m + 7) / 8;
     const long long tiles = (long long)b * p.tiles;
     if (tiles * p.heads > 0x7fffffffLL) return CLUSTEN_ERR_SHAPE;
-    split_heads(tiles, p.heads, &p.parts, &p.per_part);
-    p.total = (unsigned)(tiles * p.parts);
     p.wide_idx = p.m % 8 == 0 && reinterpret_cast<uintptr_t>(p.idx) % 16 == 0;
+    const bool m48 = p.m == kMmax && p.wide_idx;
+    // 16-bit tiles share their rows in blocks over records.  Where the records are made here, most of the time goes there: sum b128 h2 n3136 bf16
+    // 94 us, 92 in blocks, but for tables shared by a cluster 84, 97;  dot 92, 97.  Other rows than of 48 have records in the forward passes too,
+    // where shared tables lose as well (b64 h8 n784 m24 dot 37 us, 44 in blocks; in a training pass the rest makes up for it).
+    const bool blocks = sizeof(T) == 2 && p.plan && m48;
+    // (a block does little before its first head, and is large: b32 h8 n1843 52 -> 46 us (dot), 57 -> 50 (sum) with 40 warps per SM instead of 24,
+    // b128 h8 n196 unchanged; 27, 31 instead of 26, 29 with 64)
+    split_heads(tiles, p.heads, &p.parts, &p.per_part, blocks ? 40 : 24);
+    p.total = (unsigned)(tiles * p.parts);
     p.pad_cl = p.n % 8 ? p.n / 8 : -1;
     constexpr int kPer = 16 / (int)sizeof(T);
     const bool shift = p.m % 8 != 0 || (MODE == 0 && !(reinterpret_cast<uintptr_t>(p.A) % 16 == 0 && p.a_row % kPer == 0 && p.a_batch % kPer == 0 &&
                                                        p.a_head % kPer == 0));
-    const bool m48 = p.m == kMmax && p.wide_idx;
     auto pick = [&](auto plan, auto tail) {
         constexpr bool PLAN = decltype(plan)::value, TAIL = decltype(tail)::value;
-        return m48 ? (shift ? gather_groups_kernel<T, MODE, 6, MODE == 0, PLAN, TAIL> : gather_groups_kernel<T, MODE, 6, false, PLAN, TAIL>)
-                   : (shift ? gather_groups_kernel<T, MODE, 0, true, PLAN, true> : gather_groups_kernel<T, MODE, 0, false, PLAN, true>);
+        if constexpr (sizeof(T) == 2 && PLAN)
+            return blocks ? (shift ? gather_blocks_kernel<T, MODE, MODE == 0, TAIL> : gather_blocks_kernel<T, MODE, false, TAIL>)
+                          : (shift ? gather_groups_kernel<T, MODE, 0, true, PLAN, true> : gather_groups_kernel<T, MODE, 0, false, PLAN, true>);
+        else
+            return m48 ? (shift ? gather_groups_kernel<T, MODE, 6, MODE == 0, PLAN, TAIL> : gather_groups_kernel<T, MODE, 6, false, PLAN, TAIL>)
+                       : (shift ? gather_groups_kernel<T, MODE, 0, true, PLAN, true> : gather_groups_kernel<T, MODE, 0, false, PLAN, true>);
     };
     auto kernel = p.plan ? (p.pad_cl >= 0 ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{}))
                          : (p.pad_cl >= 0 ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{}));
-    const int tile = m48 ? (shift ? RowTile<T, 6, true>::kBytes : RowTile<T, 6, false>::kBytes)
-                         : (shift ? RowTile<T, 0, true>::kBytes : RowTile<T, 0, false>::kBytes);
-    const int smem = kGWarps * ((int)sizeof(GroupSmem) + tile);
+    const int rows_tile = m48 ? (shift ? RowTile<T, 6, true>::kBytes : RowTile<T, 6, false>::kBytes)
+                              : (shift ? RowTile<T, 0, true>::kBytes : RowTile<T, 0, false>::kBytes);
+    const int smem = kGWarps * ((int)sizeof(GroupSmem) + (blocks && MODE == 1 ? kScoreBytes : rows_tile)) + (blocks ? kBlockBytes : 0);
+    const unsigned grid = blocks ? (unsigned)(b * ((p.tiles + kGWarps - 1) / kGWarps) * p.parts) : (p.total + kGWarps - 1) / kGWarps;
     const int fit = resident_ctas(reinterpret_cast<const void*>(kernel), 32 * kGWarps, smem);
     if (fit < 0) return fit;
     ScopedKernelTimer timer(label, s);
-    kernel<<<(p.total + kGWarps - 1) / kGWarps, 32 * kGWarps, smem, s>>>(p);
+    kernel<<<grid, 32 * kGWarps, smem, s>>>(p);
     note_launch();
     return check_launch();
 }
