@@ -16,6 +16,9 @@
 //   softmax  maxima and sums over the 4 lanes of a row
 //   output   out^T[channel][row] = V^T x P^T: the probabilities are the B operand as they stand
 // The bias of an edge is looked up once for several heads (their table entries lie side by side).
+// Against a version with signed 64-bit look-ups, the blank logit as scalar products and output rows by shuffles: b64 h8 n1843 bf16 238 -> 226 us,
+// b256 h2 n3136 338 -> 330.  More instructions less did not help: keys and values by cp.async and ldmatrix 351 us, look-ups behind a branch 354,
+// one CTA of 20 warps per SM on neighbouring tiles (L1 hits 39 -> 51 %) 351.
 #include "group_core.cuh"
 
 namespace clusten {
@@ -90,7 +93,8 @@ __device__ __forceinline__ void stage_bias(const FusedParams& p, T* tile_b, long
     using B = BiasTile<T, RT>;
     const int R = RT > 0 ? RT : R_arg;
     const int g = lane >> 2, t = lane & 3;
-    const T* table = static_cast<const T*>(p.table) + h;
+    const char* entries = reinterpret_cast<const char*>(static_cast<const T*>(p.table) + h);
+    const unsigned row_bytes = (unsigned)(p.heads * (int)sizeof(T));      // of a table row
     if (FIRST)
         for (int z = lane; z < BH * 2 * 32; z += 32)                         // place 0 of every head and set
             store_pair(tile_b + (z >> 6) * B::kHead + ((z >> 5) & 1) * B::kSet + 2 * (z & 31), neg_inf<T>(), neg_inf<T>());
@@ -111,15 +115,16 @@ __device__ __forceinline__ void stage_bias(const FusedParams& p, T* tile_b, long
             }
             const bool ok0 = v.y == 0 && (unsigned)v.x < (unsigned)p.table_rows, ok1 = v.w == 0 && (unsigned)v.z < (unsigned)p.table_rows;
             const T none0 = RT > 0 || in0 ? Elem<T>::down(0.f) : neg_inf<T>(), none1 = RT > 0 || in1 ? Elem<T>::down(0.f) : neg_inf<T>();
-            for (int j = 0; j < nh; j += NV) {
+            for (int j = 0; j < (NV == BH ? BH : nh); j += NV) {             // (whole words: the heads at hand are all BH of them)
+                const char* first = entries + j * (int)sizeof(T);
                 HeadVec<T, NV> a, b;
 #pragma unroll
                 for (int i = 0; i < NV; ++i) {
                     a.v[i] = none0;
                     b.v[i] = none1;
                 }
-                if (ok0) a = *reinterpret_cast<const HeadVec<T, NV>*>(table + (long long)v.x * p.heads + j);
-                if (ok1) b = *reinterpret_cast<const HeadVec<T, NV>*>(table + (long long)v.z * p.heads + j);
+                if (ok0) a = *reinterpret_cast<const HeadVec<T, NV>*>(first + (unsigned long long)(unsigned)v.x * row_bytes);
+                if (ok1) b = *reinterpret_cast<const HeadVec<T, NV>*>(first + (unsigned long long)(unsigned)v.z * row_bytes);
 #pragma unroll
                 for (int i = 0; i < NV; ++i) store_pair(dst + (j + i) * B::kHead, a.v[i], b.v[i]);
             }
@@ -312,12 +317,7 @@ __device__ __forceinline__ void attend(const QueryFrag<T>& q, const char* kx, co
     }
 }
 
-__device__ __forceinline__ float2 unpack2(unsigned v, const __half*) { return __half22float2(*reinterpret_cast<const __half2*>(&v)); }
-__device__ __forceinline__ float2 unpack2(unsigned v, const __nv_bfloat16*) {
-    return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-}
-
-// The tile's query rows g, g + 8 as operands, and their products with the blank key (nullptr: none)
+// The tile's query rows g, g + 8 as operands, and their products with the blank key (nullptr: none), which stands in slot 0 of a group
 template <typename T>
 __device__ __forceinline__ void load_query(QueryFrag<T>& q, const T* y, int y_row, int rows, const T* blank_k, int g, int t, float (&blank)[2]) {
 #pragma unroll
@@ -327,17 +327,13 @@ __device__ __forceinline__ void load_query(QueryFrag<T>& q, const T* y, int y_ro
         blank[e] = 0.f;
     }
     if (blank_k) {
-        const uint4 k = __ldg(reinterpret_cast<const uint4*>(blank_k + 8 * t));
-        const unsigned kk[4] = {k.x, k.y, k.z, k.w};
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const unsigned qq[4] = {q.r[e].x, q.r[e].y, q.r[e].z, q.r[e].w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 a = unpack2(qq[i], static_cast<const T*>(nullptr)), c = unpack2(kk[i], static_cast<const T*>(nullptr));
-                blank[e] += a.x * c.x + a.y * c.y;
-            }
-        }
+        KeyRow<T> k;
+        k.v = make_uint4(0u, 0u, 0u, 0u);
+        if (g == 0) k.v = __ldg(reinterpret_cast<const uint4*>(blank_k + 8 * t));
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        group_scores(d, q, k);
+        blank[0] = __shfl_sync(kFull, d[0], 4 * g);
+        blank[1] = __shfl_sync(kFull, d[2], 4 * g);
     }
 }
 __device__ __forceinline__ void load_query(QueryFrag<float>& q, const float* y, int y_row, int rows, const float* blank_k, int g, int t, float (&blank)[2]) {
@@ -358,6 +354,8 @@ __device__ __forceinline__ void load_query(QueryFrag<float>& q, const float* y, 
 #pragma unroll
         for (int i = 0; i < 8; ++i) split_tf32(v[i], q.h[e][i], q.l[e][i]);
         blank[e] = v0.x * k0.x + v0.y * k0.y + v0.z * k0.z + v0.w * k0.w + v1.x * k1.x + v1.y * k1.y + v1.z * k1.z + v1.w * k1.w;
+        blank[e] += __shfl_xor_sync(kFull, blank[e], 1);
+        blank[e] += __shfl_xor_sync(kFull, blank[e], 2);
     }
 }
 
@@ -419,8 +417,6 @@ fused_attention_kernel(const __grid_constant__ FusedParams p) {
         RowState st;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            blank[e] += __shfl_xor_sync(kFull, blank[e], 1);
-            blank[e] += __shfl_xor_sync(kFull, blank[e], 2);
             blank[e] *= kLog2e;
             st.set[e] = p.blank_k && blank[e] > -INFINITY;   // (no reference: minus infinity, NaN)
             st.ref[e] = st.set[e] ? blank[e] : 0.f;
@@ -471,7 +467,22 @@ fused_attention_kernel(const __grid_constant__ FusedParams p) {
 #pragma unroll
                     for (int i = 0; i < 2; ++i) acc[e][mt][2 * i + j] = acc[e][mt][2 * i + j] * f + fb * bv[mt][i];
             }
-            store_set(acc[e], static_cast<T*>(p.out) + (bh * n + i0 + 8 * e) * kC, rows - 8 * e, lane);
+            T* o = static_cast<T*>(p.out) + (bh * n + i0 + 8 * e) * kC;
+            if constexpr (kF32) {
+                store_set(acc[e], o, rows - 8 * e, lane);
+            } else {
+                // a matrix has channels 8w + 2r and 8w + 2r + 1 of the rows, w = 0 .. 3 (frag_slots16): rows of 64 bytes over the head's biases, which are
+                // done with (the minus infinities in front of them stay), and a lane takes the four words of its piece
+                const T* type = nullptr;
+                const unsigned buf = smem_u32(tile_b + ((h - h0) % BH) * B::kHead + B::kPlace);
+                __syncwarp();
+                stmatrix_x4_trans(buf + row_piece(lane & 7, lane >> 3), pack2(acc[e][0][0], acc[e][0][1], type), pack2(acc[e][0][2], acc[e][0][3], type),
+                                  pack2(acc[e][1][0], acc[e][1][1], type), pack2(acc[e][1][2], acc[e][1][3], type));
+                __syncwarp();
+                if (g < rows - 8 * e)
+                    *reinterpret_cast<uint4*>(o + g * kC + 8 * t) = make_uint4(lds32(buf + row_piece(g, 0) + 4 * t), lds32(buf + row_piece(g, 1) + 4 * t),
+                                                                              lds32(buf + row_piece(g, 2) + 4 * t), lds32(buf + row_piece(g, 3) + 4 * t));
+            }
         }
     }
 }
