@@ -354,8 +354,6 @@ __device__ __forceinline__ void load_query(QueryFrag<float>& q, const float* y, 
 #pragma unroll
         for (int i = 0; i < 8; ++i) split_tf32(v[i], q.h[e][i], q.l[e][i]);
         blank[e] = v0.x * k0.x + v0.y * k0.y + v0.z * k0.z + v0.w * k0.w + v1.x * k1.x + v1.y * k1.y + v1.z * k1.z + v1.w * k1.w;
-        blank[e] += __shfl_xor_sync(kFull, blank[e], 1);
-        blank[e] += __shfl_xor_sync(kFull, blank[e], 2);
     }
 }
 
@@ -417,6 +415,10 @@ fused_attention_kernel(const __grid_constant__ FusedParams p) {
         RowState st;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
+            if (kF32) {                                      // (fp32: the lanes' shares)
+                blank[e] += __shfl_xor_sync(kFull, blank[e], 1);
+                blank[e] += __shfl_xor_sync(kFull, blank[e], 2);
+            }
             blank[e] *= kLog2e;
             st.set[e] = p.blank_k && blank[e] > -INFINITY;   // (no reference: minus infinity, NaN)
             st.ref[e] = st.set[e] ? blank[e] : 0.f;
