@@ -54,15 +54,18 @@ __device__ __forceinline__ unsigned pair16(int lo, int hi) { return (unsigned)lo
 // ----------------------------------------------------------------------------- record of a tile, from its indices
 // src = index rows of the tile (rows of them exist), n_src source rows (at most 65000).  rec, tag (kTagSpan bytes): shared
 // memory of the warp.  RT: groups per row when known at compile time (m = 8 RT; 0: R_arg);  TAIL: n_src is not a
-// multiple of 8;  wide: m is a multiple of 8 and the rows start on 16-byte boundaries.
+// multiple of 8;  wide: m is a multiple of 8 and the rows start on 16-byte boundaries;  DIVIDE: not by multiplication, which costs registers.
 // The runs y = row * R + r are read in memory order, run y = g + 8 k by the four lanes (g, t).
-template <int RT, bool TAIL>
+template <int RT, bool TAIL, bool DIVIDE = true>
 __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, int rows, int m, int R_arg, int n_src, bool wide,
                                              TileRecord& rec, unsigned char* tag, int lane) {
     constexpr int RMAX = RT > 0 ? RT : kGroupMaxR;
     const int R = RT > 0 ? RT : R_arg;
     const int g = lane >> 2, t = lane & 3;
     const int nruns = rows * R;
+    // y / R, exact for y < 128
+    const unsigned inverse = DIVIDE ? 0u : (65536u + (unsigned)R - 1u) / (unsigned)R;
+    auto row_of = [&](int y) { return DIVIDE ? y / R : (int)((unsigned)y * inverse >> 16); };
     unsigned pr[2 * RMAX];                                   // this lane's two tokens of run g + 8 k (0xffff: absent)
     unsigned out = 0u;                                       // not zero: an index out of range
     if (RT > 0 || wide) {
@@ -83,7 +86,7 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
             const int y = g + 8 * k;
             pr[k] = 0xffffffffu;
             if (y < nruns) {
-                const int row = y / R, j = 8 * (y - row * R) + 2 * t;
+                const int row = row_of(y), j = 8 * (y - row * R) + 2 * t;
                 const int64_t* q = src + (long long)row * m + j;
                 const long long a = j < m ? __ldg(q) : -1, b = j + 1 < m ? __ldg(q + 1) : -1;
                 pr[k] = pair16((unsigned long long)a < (unsigned long long)n_src ? (int)a : kSkip,
@@ -197,7 +200,7 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
 #pragma unroll
     for (int k = 0; k < 2 * RMAX; ++k) {
         const int y = g + 8 * k;
-        const int row = y / R, r = y - row * R;
+        const int row = row_of(y), r = y - row * R;
         unsigned ref;
         if (RT > 0) {
             ref = __shfl_sync(kFull, k < RT ? pr[0] : ref8, 4 * r + t);
@@ -221,7 +224,7 @@ __device__ __forceinline__ void build_record(const int64_t* __restrict__ src, in
 #pragma unroll
         for (int k = 0; k < 2 * RMAX; ++k) {
             const int y = g + 8 * k;
-            const int row = y / R, r = y - row * R;
+            const int row = row_of(y), r = y - row * R;
             if (y < nruns && (row & 7) == 0) reinterpret_cast<unsigned*>(rec.lists[row >> 3])[4 * r + t] = pr[k];
         }
     }
