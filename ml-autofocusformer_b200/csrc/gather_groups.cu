@@ -582,7 +582,7 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
 // tiles that read their own rows from L1 / L2, over records: b128 h2 n3136 bf16 dot 74 -> 66 us, sum 90 -> 72, b32 h8 n1843 fp16 60 -> 45,
 // 73 -> 50.  What is left is waiting: with its clusters on the way a block has nothing else to do, and six of them share an SM
 // (without the products the same blocks take 50 of the 66 us; the bytes that DRAM has to move, 37).
-constexpr int kBlockClusters = 40;               // with more of them (at most 35 in AutoFocusFormer's tables) each tile reads its own
+constexpr int kBlockClusters = 40;               // with more of them (35 were the most in tables of 196 to 9216 tokens) each tile reads its own
 constexpr int kBlockBytes = kBlockClusters * 512;
 
 // Scores of a tile, 16 rows of 6 pieces of 8.  The pitch is an odd number of pieces, so that 8 rows' pieces of one place lie in different

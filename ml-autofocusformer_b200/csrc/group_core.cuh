@@ -557,7 +557,6 @@ template <typename T> __device__ __forceinline__ void store_rows8(const float (&
             make_uint4(pack2(v[0], v[1], static_cast<const T*>(nullptr)), pack2(v[2], v[3], static_cast<const T*>(nullptr)),
                        pack2(v[4], v[5], static_cast<const T*>(nullptr)), pack2(v[6], v[7], static_cast<const T*>(nullptr)));
 }
-template <typename T> __device__ __forceinline__ void store_set(const float (&d)[2][4], T* out, int rows, int lane) { store_rows8(d, out, kC, rows, lane); }
 __device__ __forceinline__ unsigned byte_of(unsigned w, int i) { return __byte_perm(w, 0u, 0x4440u + i); }
 
 // ---- copies to shared memory and operands from there (16-bit); addresses are 32-bit shared ones
