@@ -130,6 +130,48 @@ def test_blank_logits_that_are_not_finite(lib):
     assert torch.isnan(got[:, 1, :16]).all() and torch.isfinite(got[:, 1, 16:]).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bfloat16", "float16"])
+def test_blank_logits_that_are_not_finite_16bit(lib, dtype):
+    """The same with minus infinity in the blank key itself."""
+    from clusten import ops
+    b, h, n, m, c = 1, 2, 200, 48, 32
+    idx = workloads.make_index("model", b, n, m, 440, DEV)
+    g = torch.Generator(device=DEV).manual_seed(441)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV).to(dtype)  # noqa: E731
+    q, k, v = rn(b, h, n, c) * c ** -0.5, rn(b, h, n, c), rn(b, h, n, c)
+    q[..., 0] = 1.0
+    blank_k, blank_v = rn(h, c), rn(h, c)
+    blank_k[0, 0] = float("-inf")
+    q[:, 1, :16, 1], blank_k[1, 1] = float("nan"), 1.0
+    got = ops.local_attention_forward(q, k, v, idx, blank_k=blank_k, blank_v=blank_v)
+    want = _chain(q[:, :1], k[:, :1], v[:, :1], idx)         # (no share for the blank token)
+    assert rel_err(got[:, :1], want) <= TOL[dtype]
+    assert torch.isnan(got[:, 1, :16]).all() and torch.isfinite(got[:, 1, 16:]).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16], ids=["float32", "bfloat16", "float16"])
+@pytest.mark.parametrize("regime,b,h,n,m", [("model", 240, 8, 241, 48), ("model", 240, 4, 241, 48), ("model", 240, 2, 240, 48), ("model", 240, 3, 241, 48),
+                                            ("model", 240, 6, 241, 48), ("shared", 240, 8, 233, 48), ("random", 240, 8, 233, 48), ("model", 240, 8, 241, 40),
+                                            ("random", 240, 6, 233, 13)])
+def test_several_heads_per_warp(lib, regime, b, h, n, m, dtype):
+    """So many tiles that a warp takes all heads (148 SMs): position biases of two or four heads at a time, the next ones' in the same place."""
+    from clusten import ops
+    c = 32
+    idx = workloads.make_index(regime, b, n, m, 450 + n, DEV)
+    g = torch.Generator(device=DEV).manual_seed(451)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV).to(dtype)  # noqa: E731
+    q, k, v = rn(b, h, n, c) * c ** -0.5, rn(b, h, n, c), rn(b, h, n, c)
+    kw = dict(pe_table=rn(111, h), blank_k=rn(h, c), blank_v=rn(h, c))
+    per_edge = dict(pe_idx=torch.randint(0, 111, (b, n, m), generator=g, device=DEV), mask=(torch.rand(b, n, m, generator=g, device=DEV) > 0.1).long())
+    got = ops.local_attention_forward(q, k, v, idx, **kw, **per_edge)
+    plain = ops.local_attention_forward(q, k, v, idx)
+    for e in (0, 117, b - 1):
+        one = slice(e, e + 1)
+        want = _chain(q[one], k[one], v[one], idx[one], **kw, **{name: t[one] for name, t in per_edge.items()})
+        assert rel_err(got[one], want) <= TOL[dtype], e
+        assert rel_err(plain[one], _chain(q[one], k[one], v[one], idx[one])) <= TOL[dtype], e
+
+
 def test_argument_checks(lib):
     p = 256
     call = lib.clusten_local_attention_forward
