@@ -655,6 +655,45 @@ __device__ __forceinline__ void dot_runs(const uint4 (&q)[2], unsigned xs, unsig
     }
 }
 
+// A list of 48 rows, no slot absent, 16-bit: all but its last two groups on their way at once.  In blocks fewer warps share an SM, with less L1, than by
+// tiles, and sum_head, two groups at a time, fell behind there: sum over records, tables shared by a cluster, b128 h2 n3136 bf16 68 us by
+// tiles, 77 in blocks, 64 so, b32 h8 n1843 39, 50, 41, b128 h8 n196 19.1, 21.8, 19.5.  (With another two groups in flight in the same way, runs and
+// rows of their own spill and take as long or longer.)  x: the head's rows at channel 4g;  tok: the list;  w, at: as for sum_head;  rows
+// that do not exist take what lies in the tile, and are not stored
+template <typename T, bool SHIFT>
+__device__ __forceinline__ void sum_list(const T* __restrict__ x, unsigned x_row, const T* w, const PairAt& at, const unsigned short* tok, int t,
+                                         float (&acc)[2][4]) {
+    const unsigned* toks = reinterpret_cast<const unsigned*>(tok) + t;
+    uint2 v[2][4];
+    auto load = [&](int u, uint2 (&d)[4]) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const unsigned tk = toks[(u + i) * 4];
+            d[2 * i] = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const char*>(x) + (unsigned long long)(tk & 0xffffu) * x_row));
+            d[2 * i + 1] = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const char*>(x) + (unsigned long long)(tk >> 16) * x_row));
+        }
+    };
+    load(0, v[0]);
+    load(2, v[1]);
+    cp_async_wait<0>();                                      // (the weights)
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kBlockR; u += 2) {
+        uint2 (&d)[4] = v[(u >> 1) & 1];
+        unsigned a[2][4], b[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const T* q = w + 64 * (u + i + 1);
+            if (SHIFT) b[i] = __funnelshift_r(*reinterpret_cast<const unsigned*>(q + at.first), *reinterpret_cast<const unsigned*>(q + at.second), at.bits);
+            else b[i] = *reinterpret_cast<const unsigned*>(q);
+        }
+        frag_channels16(a, d[0], d[1], d[2], d[3]);
+        if (u + 4 < kBlockR) load(u + 4, d);
+        mma16(acc[0], a[0], b, static_cast<const T*>(nullptr));
+        mma16(acc[1], a[1], b, static_cast<const T*>(nullptr));
+    }
+}
+
 // A tile by itself, 16-bit, its record unpacked (the weights of the first head are on their way): as in gather_groups_kernel
 template <typename T, int MODE, bool SHIFT, bool TAIL>
 __device__ __forceinline__ void gather_tile(const GatherGroupsParams& p, GroupSmem& sm, T* tile, const T* A, const T* X, const int64_t* src, int b, int i0, int rows,
@@ -706,7 +745,7 @@ __device__ __forceinline__ void gather_tile(const GatherGroupsParams& p, GroupSm
                     if (kind == kRecSame) {
                         const unsigned short* tok = sm.tok + e * kGroupMaxM;
                         if (holes) sum_head<Pick<false, true>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
-                        else sum_head<Pick<false, false>, T, SHIFT, 1, Tile::kSet>(Xh, p.x_row, we, at, map, sm, tok, U0, -1, n, t, acc);
+                        else sum_list<T, SHIFT>(Xh, p.x_row, we, at[0], tok, t, acc[0]);
                     } else {
                         for (int first = 8 * e, U; first < min(rows, 8 * e + 8);) {
                             first += load_piece<kBlockR>(src, first, rows, m, n, p.wide_idx != 0, sm, lane, &U);
