@@ -951,7 +951,11 @@ int gather_groups_t(const char* label, GatherGroupsParams p, int b, cudaStream_t
     // 16-bit tiles share their rows in blocks over records.  Where the records are made here, most of the time goes there: sum b128 h2 n3136 bf16
     // 94 us, 92 in blocks, but for tables shared by a cluster 84, 97;  dot 92, 97.  Other rows than of 48 have records in the forward passes too,
     // where shared tables lose as well (b64 h8 n784 m24 dot 37 us, 44 in blocks; in a training pass the rest makes up for it).
-    const bool blocks = sizeof(T) == 2 && p.plan && m48;
+    // Dot products only from 128 (tile, head) pairs per SM on: a block has barriers, and its clusters on the way, in front of few products (QK forward over records,
+    // us by tiles / in blocks: b128 h8 n196 16.8 / 17.4, b16 h2 n3136 10.3 / 11.3, b4 h2 n9216 8.1 / 10.1, b4 h4 n784 4.4 / 4.8; above:
+    // b64 h8 n784 33 / 30, b32 h8 n1843 52 / 39).  Sums gain at every size (b128 h8 n196 22 / 19, b4 h2 n9216 11.8 / 10.9, b1 h8 n196 5.0 / 4.3).
+    constexpr bool kBlocks = sizeof(T) == 2;
+    const bool blocks = kBlocks && p.plan && m48 && (MODE == 0 || tiles * p.heads >= 128LL * sm_count());
     // (a block does little before its first head, and is large: b32 h8 n1843 52 -> 46 us (dot), 57 -> 50 (sum) with 40 warps per SM instead of 24,
     // b128 h8 n196 unchanged; 27, 31 instead of 26, 29 with 64)
     split_heads(tiles, p.heads, &p.parts, &p.per_part, blocks ? 40 : 24);
@@ -962,12 +966,12 @@ int gather_groups_t(const char* label, GatherGroupsParams p, int b, cudaStream_t
                                                        p.a_head % kPer == 0));
     auto pick = [&](auto plan, auto tail) {
         constexpr bool PLAN = decltype(plan)::value, TAIL = decltype(tail)::value;
-        if constexpr (sizeof(T) == 2 && PLAN)
-            return blocks ? (shift ? gather_blocks_kernel<T, MODE, MODE == 0, TAIL> : gather_blocks_kernel<T, MODE, false, TAIL>)
-                          : (shift ? gather_groups_kernel<T, MODE, 0, true, PLAN, true> : gather_groups_kernel<T, MODE, 0, false, PLAN, true>);
-        else
-            return m48 ? (shift ? gather_groups_kernel<T, MODE, 6, MODE == 0, PLAN, TAIL> : gather_groups_kernel<T, MODE, 6, false, PLAN, TAIL>)
-                       : (shift ? gather_groups_kernel<T, MODE, 0, true, PLAN, true> : gather_groups_kernel<T, MODE, 0, false, PLAN, true>);
+        if constexpr (kBlocks && PLAN) {
+            if (blocks) return shift ? gather_blocks_kernel<T, MODE, MODE == 0, TAIL> : gather_blocks_kernel<T, MODE, false, TAIL>;
+            if constexpr (MODE == 0) return shift ? gather_groups_kernel<T, MODE, 0, true, PLAN, true> : gather_groups_kernel<T, MODE, 0, false, PLAN, true>;
+        }
+        return m48 ? (shift ? gather_groups_kernel<T, MODE, 6, MODE == 0, PLAN, TAIL> : gather_groups_kernel<T, MODE, 6, false, PLAN, TAIL>)
+                   : (shift ? gather_groups_kernel<T, MODE, 0, true, PLAN, true> : gather_groups_kernel<T, MODE, 0, false, PLAN, true>);
     };
     auto kernel = p.plan ? (p.pad_cl >= 0 ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{}))
                          : (p.pad_cl >= 0 ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{}));

@@ -177,3 +177,29 @@ def test_values_that_are_not_finite(lib, kind, layout, dtype):
         assert x[:, tile(w, width)].all(), name
         if kind == "model" and width == 8:
             assert torch.equal(x, w), name
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bfloat16", "float16"])
+@pytest.mark.parametrize("layout", ["plain", "views"])
+@pytest.mark.parametrize("kind", ["model", "shared", "random", "unnamed", "outside", "twice", "far"])
+@pytest.mark.parametrize("b,h,n", [(8, 16, 2368), (8, 16, 2352), (4, 3, 357), (1, 2, 45)])
+def test_over_records_and_without(lib, kind, b, h, n, layout, dtype):
+    """Forward passes over records (blocks; dot products from 128 tiles and heads per SM on, 8 x 16 x 148 on 148 SMs) and with records made in the kernel,
+    tile by tile: the same products in the same order."""
+    from clusten import _lib
+    m = 48
+    idx = _table(kind if kind in ("model", "shared", "random", "unnamed") else "shared" if kind == "outside" else "model", b, n, m, 770 + n)
+    if kind == "outside":
+        idx[:, ::5, 3], idx[:, 1::7, m - 1] = -1, n + 2
+    elif kind == "twice":                                     # every 37th row names its first cluster twice
+        idx[:, ::37, 8:16] = idx[:, ::37, 0:8]
+    elif kind == "far":                                       # tiles in any order: blocks of more clusters than they hold, next to others
+        tile = torch.arange(n, device=DEV) // 16
+        order = torch.where(tile % 8 < 4, tile, (7 * tile + 3) % (n // 16)).clamp_(max=n // 16 - 1)
+        idx = idx[:, order * 16 + torch.arange(n, device=DEV) % 16].contiguous()
+    q, k, attn, v = _operands(b, h, n, m, layout, dtype, 771)[:4]
+    host = _lib.host()
+    for over, without in ((host.qk_forward(q, k, idx, True), host.qk_forward(q, k, idx, False)),
+                          (host.av_forward(attn, v, idx, True), host.av_forward(attn, v, idx, False))):
+        assert over[1] is not None and without[1] is None
+        assert torch.equal(over[0], without[0])
