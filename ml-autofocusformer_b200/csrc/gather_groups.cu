@@ -409,13 +409,15 @@ __device__ __forceinline__ void store_rows(const T* tile, T* __restrict__ out, i
 // SHIFT: the rows of the weights (sum) or scores (dot, LinearRows) do not start on 16-byte boundaries;  PLAN: the records are there;
 // TAIL: the last cluster is padded
 // CTAs per SM, measured for b128 h2 n3136.  dot: fp32 over records 7 (0.115 ms a call, 0.130 with 5), 5 where the records are made here
-// (b4 h2 n9216 22 us, 24 with 6); 16-bit 4, without spills (b128 h8 n196 22.8 us, 28.3 with 6).  sum: fp32 over records 5, 6 where they are
-// made here (shared tables 134 us, 138 with 5; b128 h8 n196 45, 50 with 5), 16-bit 7.
+// (b4 h2 n9216 22 us, 24 with 6); 16-bit 4, without spills (91 us, 102 with 6; b128 h8 n196 23.2, 25.2; shared tables 99, 94).  sum: fp32 over records
+// 5, 6 where they are made here (shared tables 134 us, 138 with 5; b128 h8 n196 45, 50 with 5), 16-bit 7.
 template <typename T, int MODE, bool PLAN> constexpr int gather_ctas() {
     if (MODE == 1) return sizeof(T) == 4 ? (PLAN ? 7 : 5) : 4;
     return sizeof(T) == 4 ? (PLAN ? 5 : 6) : 7;
 }
-constexpr int kBlockCtas = 6;                    // blocks (below): dot 66 us, sum 72 (5: 68, 72; 7: 62, 76; tables shared by a cluster 92, 97, 110)
+// Blocks (below), us with 6 (5, 7), b128 h2 n3136 bf16: dot 61 (64, 59), sum 62 (66, 62), of the model's views 70 (75, 72); b64 h8 n784 30 (33, 30), 31 (36, 34);
+// tables shared by a cluster, tile by tile inside: dot 82 (76, 87), b32 h8 n1843 53 (46, 63), sum 63 (67, 65), 41 (41, 39)
+constexpr int kBlockCtas = 6;
 template <typename T, int MODE, int RT, bool SHIFT, bool PLAN, bool TAIL>
 __global__ void __launch_bounds__(32 * kGWarps, (gather_ctas<T, MODE, PLAN>()))
 gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
@@ -579,9 +581,9 @@ gather_groups_kernel(const __grid_constant__ GatherGroupsParams p) {
 // ----------------------------------------------------------------------------- blocks of 64 rows, 16-bit
 // A CTA's four tiles are consecutive.  When all of them have whole clusters, the distinct ones among them -- 25 where the tiles by themselves
 // have 4 x 13 -- go to shared memory once per head, and the products read them there (sum: ldmatrix.trans, dot: 16-byte loads).  Against
-// tiles that read their own rows from L1 / L2, over records: b128 h2 n3136 bf16 dot 74 -> 66 us, sum 90 -> 72, b32 h8 n1843 fp16 60 -> 45,
-// 73 -> 50.  What is left is waiting: with its clusters on the way a block has nothing else to do, and six of them share an SM
-// (without the products the same blocks take 50 of the 66 us; the bytes that DRAM has to move, 37).
+// tiles that read their own rows from L1 / L2, over records: b128 h2 n3136 bf16 dot 70 -> 61 us, sum of the model's views 88 -> 70,
+// b32 h8 n1843 52 -> 39, 65 -> 45.  What is left is waiting: with its clusters on the way a block has nothing else to do, and six of them
+// share an SM (issue slots 45 and 57 % busy, L1 68 and 58 %, DRAM 42 % of its rate).
 constexpr int kBlockClusters = 40;               // with more of them (35 were the most in tables of 196 to 9216 tokens) each tile reads its own
 constexpr int kBlockBytes = kBlockClusters * 512;
 
@@ -694,7 +696,9 @@ __device__ __forceinline__ void sum_list(const T* __restrict__ x, unsigned x_row
     }
 }
 
-// A tile by itself, 16-bit, its record unpacked (the weights of the first head are on their way): as in gather_groups_kernel
+// A tile by itself, 16-bit, its record unpacked (the weights of the first head are on their way): as in gather_groups_kernel, which has a body of its own,
+// because the compiler schedules one that serves both kernels worse (fp32 dot b128 h2 n3136 174 -> 185 us, bf16 sum b64 h2 n3136 m40 41 -> 44).
+// What changes in one of them changes in the other: the tests compare the two bit by bit
 template <typename T, int MODE, bool SHIFT, bool TAIL>
 __device__ __forceinline__ void gather_tile(const GatherGroupsParams& p, GroupSmem& sm, T* tile, const T* A, const T* X, const int64_t* src, int b, int i0, int rows,
                                             int h0, int h1, int lane) {
@@ -950,14 +954,16 @@ int gather_groups_t(const char* label, GatherGroupsParams p, int b, cudaStream_t
     const bool m48 = p.m == kMmax && p.wide_idx;
     // 16-bit tiles share their rows in blocks over records.  Where the records are made here, most of the time goes there: sum b128 h2 n3136 bf16
     // 94 us, 92 in blocks, but for tables shared by a cluster 84, 97;  dot 92, 97.  Other rows than of 48 have records in the forward passes too,
-    // where shared tables lose as well (b64 h8 n784 m24 dot 37 us, 44 in blocks; in a training pass the rest makes up for it).
+    // where shared tables lose as well (b64 h8 n784 m24 dot 37 us, 44 in blocks).  Which kind a table is, the host does not know: what blocks
+    // cannot serve goes tile by tile inside, and is slower there than in the kernel of tiles where rows have little in common (sum by tiles / here:
+    // tiles in any order, blocks of more than 40 clusters, b128 h2 n3136 80 / 89; random rows b32 h8 n1843 229 / 260, b4 h4 n784 19.5 / 20.2).
     // Dot products only from 128 (tile, head) pairs per SM on: a block has barriers, and its clusters on the way, in front of few products (QK forward over records,
     // us by tiles / in blocks: b128 h8 n196 16.8 / 17.4, b16 h2 n3136 10.3 / 11.3, b4 h2 n9216 8.1 / 10.1, b4 h4 n784 4.4 / 4.8; above:
     // b64 h8 n784 33 / 30, b32 h8 n1843 52 / 39).  Sums gain at every size (b128 h8 n196 22 / 19, b4 h2 n9216 11.8 / 10.9, b1 h8 n196 5.0 / 4.3).
     constexpr bool kBlocks = sizeof(T) == 2;
     const bool blocks = kBlocks && p.plan && m48 && (MODE == 0 || tiles * p.heads >= 128LL * sm_count());
-    // (a block does little before its first head, and is large: b32 h8 n1843 52 -> 46 us (dot), 57 -> 50 (sum) with 40 warps per SM instead of 24,
-    // b128 h8 n196 unchanged; 27, 31 instead of 26, 29 with 64)
+    // (a block does little before its first head, and is large: b32 h8 n1843 44 -> 39 us (dot), 47 -> 41 (sum) with 40 warps per SM instead of 24,
+    // b128 h8 n196 sum 18.8 with both; 20.9 with 64)
     split_heads(tiles, p.heads, &p.parts, &p.per_part, blocks ? 40 : 24);
     p.total = (unsigned)(tiles * p.parts);
     p.pad_cl = p.n % 8 ? p.n / 8 : -1;

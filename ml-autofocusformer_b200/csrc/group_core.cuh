@@ -570,9 +570,6 @@ __device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], unsigned a) 
 __device__ __forceinline__ void ldmatrix_x2_trans(unsigned (&r)[2], unsigned a) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], unsigned a) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
-}
 __device__ __forceinline__ void stmatrix_x4(unsigned a, unsigned r0, unsigned r1, unsigned r2, unsigned r3) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }

@@ -119,10 +119,13 @@ bool av_backward_takes(const Tensor& g, const Tensor& a, const Tensor& v, const 
 // Records of a table (clusten_groups_build) for one forward call.  They are made from the indices as they are now and never kept
 // for a later forward call: a table can change without a trace that could be checked (a replayed graph, another library's kernel),
 // and a buffer of another stream or of a capture need not have been written yet.
-// When they pay within the call -- QK / AV, us with the build against without: not for rows of 48, which the kernels
-// analyse at compile-time sizes (b128 h2 n3136 bf16 99 / 118 against 88 / 110, b64 h8 n196 14 / 19 against 17 / 20);  other
-// rows from 2 M scores on (b256 h16 n49 m49 39 / 36 against 46 / 41, b64 h8 n784 m24 fp32 74 / 83 against 84 / 87; below:
-// b16 h16 n49 m49 13 / 13 against 12 / 12, b4 h8 n784 m24 8 / 10 against 7 / 9).
+// When they pay within the call -- QK / AV, us with the build against without: not for rows of 48, which the kernels analyse at compile-time
+// sizes.  With two heads nothing is gained (b128 h2 n3136 bf16 93 / 94 against 91 / 93, tables shared by a cluster 112 / 93 against 99 / 83);
+// with eight it depends on what the host does not know: whole clusters gain in 16 bits (b32 h8 n1843 47 / 49 against 56 / 58, b64 h8 n784 36 / 37
+// against 42 / 50, b128 h8 n196 22 / 24 against 23 / 27), shared tables lose (60 / 48 against 55 / 45, 45 / 37 against 46 / 41, 23 / 24 against
+// 23 / 25).  Other rows from 2 M scores on (b256 h16 n49 m49 bf16 38 / 37 against 46 / 42, b64 h8 n784 m24 whole clusters bf16 38 / 42 against 41 / 45,
+// fp32 75 / 73 against 82 / 74, shared 64 / 63 against 79 / 57, b64 h2 n3136 m40 shared bf16 70 / 65 against 69 / 63; below: b4 h8 n784 m24 bf16
+// 9 / 10 against 8 / 9).
 constexpr int64_t kRecordsMinScores = int64_t(1) << 21;
 OptTensor records(const Tensor& idx, int heads, int n, bool wanted, int& status) {
     status = CLUSTEN_OK;

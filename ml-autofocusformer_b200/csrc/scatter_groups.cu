@@ -97,7 +97,7 @@ __device__ __forceinline__ void step_rows(float (&acc)[2][4], const T* const (&r
 // cp.async, kSDepth - 1 steps ahead and across the warp's heads, and come back as operands by ldmatrix.trans.  The entries
 // behind the last one (place 0) are filled with zeros without a look at memory.  Against rows and weights that went from L1 straight
 // into operand registers: b128 h2 n3136 bf16 121 -> 97 us, b32 h8 n1843 fp16 111 -> 63, b128 h8 n196 bf16 62 -> 34 (in the last two
-// one more walk over the padded cluster's list instead of one per padded slot).  Bound by the L1 (83 % busy): a row of X or of
+// one more walk over the padded cluster's list instead of one per padded slot).  Bound by the L1 (83 % busy, b64 h2 n3136): a row of X or of
 // weights is a line of its own.
 constexpr int kSDepth = 2;                        // (3: the same times with 20 % more shared memory; 4: b128 h2 n3136 bf16 120 us, for want of L1)
 template <bool SHIFT> struct RunsStage {
@@ -475,7 +475,8 @@ int launch_scatter_groups(const char* label, int dtype, const void* W, const voi
     p.heads = h;  p.n = n;  p.m = m;
     const long long tiles = (long long)b * inv.ntiles;
     if (tiles * h > 0x7fffffffLL) return CLUSTEN_ERR_SHAPE;
-    // 16-bit warps have little to read before the first head: more of them (b32 h8 n1843 fp16 63 us, 70 with 24 per SM; b128 h8 n196 bf16 33, 37)
+    // 16-bit warps have little to read before the first head: more of them (b32 h8 n1843 fp16 63 us, 70 with 24 per SM; b128 h8 n196 bf16 33, 37).  The ordinary
+    // index, whose warps go target by target, gains most: d_query and d_key of random tables b32 h8 n1843 bf16 1707 us, 2456 with 24, b64 h8 n784 2061, 3128
     split_heads(tiles, h, &p.parts, &p.per_part, dtype == CLUSTEN_F32 ? 24 : 64);
     p.total = (unsigned)(tiles * p.parts);
     while ((1ull << p.m_shift) < (unsigned)m) ++p.m_shift;
