@@ -10,7 +10,7 @@
 // element.  Rows are taken in the row order, so the two rows of a warp and the rows of neighbouring warps share
 // most of their neighbours and find them in L1.  No shared memory and 64 registers: 32 warps per SM, against 12
 // for the tiled kernel (wf_tiles_kernel), whose staging, de-duplication and three-pass TF32 products cost more
-// instruction slots than these 16 FMAs per neighbour.  16-bit inputs have kernels of their own below.
+// instruction slots than these 16 FMAs per neighbour.  16-bit inputs take it where few weights share a feature row; else kernels of their own below.
 #include "group_core.cuh"
 #include "tiled.cuh"
 
@@ -491,8 +491,13 @@ static int wf_forward_direct_ic(const char* label, int ic, const WfDirectParams&
 int launch_wf_forward_direct(const char* label, int dtype, const void* W, const void* F, const int64_t* idx,
                              const int* order, void* out, int b, int n_out, int n, int m, int ic, int c,
                              cudaStream_t s) {
-    if (dtype != CLUSTEN_F32) {
-        if ((long long)b * n_out > 0x7fffffffLL) return CLUSTEN_ERR_SHAPE;
+    // 16-bit: the tensor-core kernel does the work of 48 slots and 8 weights whatever there are, and more of it per row before the first channels; the walk's work
+    // grows with m and ic.  us, walk / tensor cores: c 64 (b128 n3136 n_out 784) ic 1 m 48 60 / 95, m 24 40 / 93, ic 2 79 / 94, 54 / 85, ic 4 111 / 103,
+    // 75 / 89;  c 256 ic 1 232 / 264, 153 / 245, ic 2 295 / 257, 201 / 218, ic 4 450 / 281, 299 / 239;  c 512 m 48 ic 1 462 / 494, ic 2 596 / 482.
+    // The walk needs warps (half a one per row): b128 n_out 50 c 64 ic 1 6.8 / 9.1, b8 n_out 196 5.1 / 4.7, c 512 18.9 / 13.3
+    const bool walk = m * ic <= (c == 64 ? 96 : 48) && (long long)b * n_out >= 32LL * sm_count();
+    if (dtype != CLUSTEN_F32 && (long long)b * n_out > 0x7fffffffLL) return CLUSTEN_ERR_SHAPE;
+    if (dtype != CLUSTEN_F32 && !walk) {
         WfFw16Params p{};
         p.W = W;  p.F = F;  p.out = out;  p.idx = idx;  p.order = order;
         p.n_out = n_out;  p.n = n;  p.m = m;  p.c = c;  p.total = (unsigned)b * n_out;
@@ -502,7 +507,12 @@ int launch_wf_forward_direct(const char* label, int dtype, const void* W, const 
     p.W = W;  p.F = F;  p.out = out;  p.idx = idx;  p.order = order;
     p.batch = b;  p.n_out = n_out;  p.n = n;  p.m = m;  p.c = c;
     if ((long long)b * ((n_out + 1) / 2) > 0x7fffffffLL) return CLUSTEN_ERR_SHAPE;
-    return wf_forward_direct_ic<float>(label, ic, p, s);
+    switch (dtype) {
+        case CLUSTEN_F32: return wf_forward_direct_ic<float>(label, ic, p, s);
+        case CLUSTEN_F16: return wf_forward_direct_ic<__half>(label, ic, p, s);
+        case CLUSTEN_BF16: return wf_forward_direct_ic<__nv_bfloat16>(label, ic, p, s);
+        default: return CLUSTEN_ERR_DTYPE;
+    }
 }
 
 int launch_wf_dweights_direct(const char* label, int dtype, const void* F, const void* G, const int64_t* idx, const int* order,
